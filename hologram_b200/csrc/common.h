@@ -267,6 +267,9 @@ int32_t holo_launch_matmul_add_activation(holo_b200_ctx* ctx, const void* a, con
                                           uint8_t dtype, uint8_t fused_act, const void* residual);
 int32_t holo_launch_matmul_multi(holo_b200_ctx* ctx, const void* a, const void* b, uint32_t m, uint32_t k, uint32_t n,
                                  uint8_t dtype, const HoloMatmulSeg* segs, uint32_t nseg);
+// gemm_cell.cu: the reference's per-cell recurrence; `act` a LUT id or -1, `add_first`: act(A . B + residual)
+int32_t holo_launch_matmul_cell(holo_b200_ctx* ctx, const void* a, const void* b, void* out, const uint16_t* table, int act, const void* residual, uint32_t m,
+                                uint32_t k, uint32_t n, uint8_t dtype, int add_first);
 // linear.cu
 struct HoloLinearSegArgs {
     void* out;

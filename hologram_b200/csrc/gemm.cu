@@ -1,51 +1,6 @@
-// bf16 / f16 matmul with the reference's epilogues: the per-cell kernel and the launchers. The tensor-core kernels
-// are in gemm_kernels.cuh.
+// bf16 / f16 matmul with the reference's epilogues: the launchers. The tensor-core kernels are in gemm_kernels.cuh, the
+// per-cell recurrence in gemm_cell.cu.
 #include "gemm_kernels.cuh"
-
-namespace {
-
-// Shapes the tensor-core path cannot take (row pitches that are not 16-byte multiples,
-// unaligned bases), tiny problems and every f32 product: one thread per output cell running the
-// reference's own per-cell recurrence, an ascending-k fused multiply-add chain (mul-then-add in
-// the n % 8 column tail, cpu/simd.rs:746-799) -- bit-identical to the CPU kernel. For f32 the
-// fused activation is the scalar function itself (no table exists for 32-bit patterns).
-// `add_first` (MatMulAddActivation, cpu/float_kernels.rs:899-938): the residual is added before the activation and
-// nothing is narrowed between the two; for 16-bit dtypes the product itself is narrowed once, as the matmul stores it.
-__global__ void matmul_cell_kernel(const void* __restrict__ a, const void* __restrict__ b, void* __restrict__ out,
-                                   const uint16_t* __restrict__ table, int act, const void* __restrict__ residual, uint32_t m,
-                                   uint32_t k, uint32_t n, int dtype, int add_first) {
-    holo_pdl_trigger();
-    holo_pdl_wait();
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
-    if (j >= n || i >= m) return;
-    const bool fused = j < n - (n % 8);
-    float acc = 0.0f;
-    for (uint32_t kk = 0; kk < k; ++kk) {
-        float av = holo::load_float(a, (uint64_t)i * k + kk, dtype), bv = holo::load_float(b, (uint64_t)kk * n + j, dtype);
-        acc = fused ? __fmaf_rn(av, bv, acc) : __fadd_rn(acc, __fmul_rn(av, bv));
-    }
-    const uint64_t idx = (uint64_t)i * n + j;
-    if (add_first) {
-        if (dtype == HOLO_DTYPE_F32) {
-            acc = __fadd_rn(acc, reinterpret_cast<const float*>(residual)[idx]);
-            reinterpret_cast<float*>(out)[idx] = holo::lut_act_ref(act, acc);
-        } else {
-            const float v = __fadd_rn(holo::widen16(holo::narrow16(acc, dtype), dtype), holo::widen16(reinterpret_cast<const uint16_t*>(residual)[idx], dtype));
-            reinterpret_cast<uint16_t*>(out)[idx] = holo::narrow16(holo::lut_act_ref(act, v), dtype);
-        }
-        return;
-    }
-    if (dtype == HOLO_DTYPE_F32) {
-        if (act >= 0) acc = holo::lut_act_ref(act, acc);
-        if (residual) acc = __fadd_rn(acc, reinterpret_cast<const float*>(residual)[idx]);
-        reinterpret_cast<float*>(out)[idx] = acc;
-    } else {
-        const uint16_t* res16 = reinterpret_cast<const uint16_t*>(residual);
-        reinterpret_cast<uint16_t*>(out)[idx] = dtype == HOLO_DTYPE_F16 ? epilogue_elem<true>(acc, table, res16, idx) : epilogue_elem<false>(acc, table, res16, idx);
-    }
-}
-
-}  // namespace
 
 static int lut_id_of_fused(uint8_t fused_act) {
     return fused_act == HOLO_FUSED_GELU ? HOLO_LUT_GELU : fused_act == HOLO_FUSED_SILU ? HOLO_LUT_SILU
@@ -71,11 +26,7 @@ int32_t holo_launch_matmul(holo_b200_ctx* ctx, const void* a, const void* b, voi
 
 int32_t holo_launch_matmul_add_activation(holo_b200_ctx* ctx, const void* a, const void* b, void* out, uint32_t m, uint32_t k, uint32_t n,
                                           uint8_t dtype, uint8_t fused_act, const void* residual) {
-    if (m > 65535) return holo_fail(HOLO_ERR_UNSUPPORTED_OP, "unsupported op: matmul m %u on the per-cell path", m);
-    HOLO_CUDA(holo_launch_kernel(ctx, matmul_cell_kernel, dim3((n + 127) / 128, m), dim3(128), 0, 1, a, b, out, (const uint16_t*)nullptr,
-                                 lut_id_of_fused(fused_act), residual, m, k, n, (int)dtype, 1));
-    ctx->launches++;
-    return HOLO_OK;
+    return holo_launch_matmul_cell(ctx, a, b, out, nullptr, lut_id_of_fused(fused_act), residual, m, k, n, dtype, 1);
 }
 
 // C[:, segment i] = epilogue_i(A . B[:, segment i]) for 1..3 column segments of one [k, n] B.
@@ -147,15 +98,7 @@ int32_t holo_launch_matmul_multi(holo_b200_ctx* ctx, const void* a, const void* 
         HOLO_TRY(holo_launch_matmul_multi(ctx, a, b, m, k, n, dtype, &plain, 1));
         return holo_all_reduce_add(ctx, segs[0].out, segs[0].residual, segs[0].out, (uint64_t)m * n, dtype);
     }
-    if (cell_path) {
-        dim3 grid((n + 127) / 128, m);
-        if (m > 65535) return holo_fail(HOLO_ERR_UNSUPPORTED_OP, "unsupported op: matmul m %u on the per-cell path", m);
-        HOLO_CUDA(holo_launch_kernel(ctx, matmul_cell_kernel, dim3(grid), dim3(128), 0, 1, a, b, out, table,
-                                     segs[0].fused_act ? lut_id_of_fused(segs[0].fused_act) : -1, residual, m, k, n, (int)dtype, 0));
-        HOLO_CUDA(cudaGetLastError());
-        ctx->launches++;
-        return HOLO_OK;
-    }
+    if (cell_path) return holo_launch_matmul_cell(ctx, a, b, out, table, segs[0].fused_act ? lut_id_of_fused(segs[0].fused_act) : -1, residual, m, k, n, dtype, 0);
     const uint32_t kblocks = (k + BK - 1) / BK, mtiles = (m + BM - 1) / BM;
     // Compute-bound shapes (at least one 128 x 256 tile per SM): the persistent kernel.
     {

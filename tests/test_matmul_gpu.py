@@ -179,6 +179,27 @@ def test_f32_matmul_is_the_reference_recurrence(backend, m, k, n):
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
 
 
+@pytest.mark.parametrize("dtype", [kc.DTYPE_F32, BF, kc.DTYPE_F16])
+@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (1, 33, 41), (3, 31, 1003), (5, 100, 64), (16, 37, 531), (33, 65, 130), (129, 7, 8 * 37), (200, 70, 2055),
+                                   (500, 50, 771), (1025, 36, 1801), (4, 96, 7)])
+def test_every_tile_of_the_per_cell_kernel_is_bit_exact(backend, dtype, m, k, n):
+    # edges of the tiles and of the k steps, pitches that are multiples of four elements and that are not, columns of the
+    # multiply-then-add tail alone and beside full tiles, chains whose sums are -0 and subnormal
+    if dtype != kc.DTYPE_F32 and k % 8 == 0 and n % 8 == 0:
+        pytest.skip("tensor-core shape")
+    rng = np.random.default_rng(m + 3 * k + 5 * n)
+    a, b, r = rng.standard_normal(m * k, dtype=np.float32), rng.standard_normal(k * n, dtype=np.float32), rng.standard_normal(m * n, dtype=np.float32)
+    if dtype == kc.DTYPE_F32:
+        a[:k] = np.float32(-1e-30)
+        b[::n] = np.float32(1e-30)
+    else:
+        narrow = orc.f32_to_bf16_rne if dtype == BF else (lambda x: x.astype(np.float16).view(np.uint16))
+        a, b, r = narrow(a), narrow(b), narrow(r)
+    bits = np.uint32 if dtype == kc.DTYPE_F32 else np.uint16
+    assert np.array_equal(run_dt(backend, a, b, m, k, n, dtype).view(bits), orc.matmul(a, b, m, k, n, dtype).view(bits))
+    assert np.array_equal(run_dt(backend, a, b, m, k, n, dtype, residual=r).view(bits), orc.matmul(a, b, m, k, n, dtype, residual=r).view(bits))
+
+
 @pytest.mark.parametrize("dtype,m,k,n,act", [(kc.DTYPE_F32, 5, 64, 24, kc.FUSED_GELU), (kc.DTYPE_F32, 3, 33, 17, kc.FUSED_SILU),
                                              (BF, 4, 128, 40, kc.FUSED_TANH), (kc.DTYPE_F16, 6, 72, 16, kc.FUSED_SIGMOID)])
 def test_matmul_add_activation_is_the_three_calls(backend, dtype, m, k, n, act):
