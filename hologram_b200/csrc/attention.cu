@@ -847,6 +847,11 @@ uint32_t persistent_ctas(uint32_t tiles_per_plane, uint32_t planes, int sm_count
 }  // namespace
 
 int32_t holo_launch_decode_attention(holo_b200_ctx* ctx, const HoloAttnArgs& a) {
+    if (!getenv("HOLO_ATTN_FORCE_GENERIC")) {
+        bool taken = false;
+        HOLO_TRY(holo_try_attention_tile(ctx, a, &taken));
+        if (taken) return HOLO_OK;
+    }
     const uint32_t G = a.h / a.hkv, planes = a.b * a.hkv;
     const bool aligned = (((uintptr_t)a.k_past | (uintptr_t)a.v_past | (uintptr_t)a.k_past_s | (uintptr_t)a.v_past_s |
                            (uintptr_t)a.k_new | (uintptr_t)a.v_new) & 15u) == 0;

@@ -229,6 +229,8 @@ struct HoloAttnArgs {
     bool all_new;     // scalar-mask form without the causal law: query row i sees every chunk row (legacy non-causal Attention)
 };
 int32_t holo_launch_decode_attention(holo_b200_ctx* ctx, const HoloAttnArgs& a);
+// attention_rows.cu: whole 16-bit sequences; *taken false: the shape is not one it serves
+int32_t holo_try_attention_tile(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool* taken);
 // gemm.cu
 int32_t holo_launch_matmul(holo_b200_ctx* ctx, const void* a, const void* b, void* out, uint32_t m, uint32_t k,
                            uint32_t n, uint8_t dtype, uint8_t fused_act, const void* residual, bool b_constant = false);

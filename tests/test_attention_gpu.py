@@ -290,3 +290,60 @@ def test_legacy_attention_prefill_form(backend):
             got, want = orc.bf16_to_f32(got), orc.bf16_to_f32(want)
         assert norm_max_err(got, want) <= (1e-2 if dt == BF else 2e-4), (idx, norm_max_err(got, want))
         ws.close()
+
+
+def run_attention(backend, q, k, v, b, h, kv, s, d, causal, dtype, scale_bits=0):
+    ws = hb.DeviceWorkspace(backend, 4)
+    for i, x in enumerate((q, k, v)):
+        ws.put(i, x)
+    ws.alloc(3, q.nbytes)
+    backend.dispatch(kc.KernelCall.Attention(kc.AttentionCall(kc.rb(0), kc.rb(1), kc.rb(2), kc.rb(3), b, h, s, d, kv if kv != h else 0, int(causal), scale_bits, dtype)), ws)
+    out = ws.read(3, q.nbytes, q.dtype)
+    ws.close()
+    return out
+
+
+def attention_inputs(b, h, kv, s, d, dtype, seed, sigma=1.0):
+    rng = np.random.default_rng(seed)
+    x = [rng.standard_normal(n).astype(np.float32) for n in (b * h * s * d, b * kv * s * d, b * kv * s * d)]
+    x[0] *= sigma
+    return x if dtype == F32 else [orc.f32_to_bf16_rne(t) if dtype == BF else t.astype(np.float16).view(np.uint16) for t in x]
+
+
+def wide(x, dtype):
+    return x if dtype == F32 else orc.bf16_to_f32(x) if dtype == BF else x.view(np.float16).astype(np.float32)
+
+
+# one unit in the last place of the output: bf16 is truncated, f16 rounded; f32 sums stay two orders below what they are held to
+ATTENTION_TOL = {BF: 2.0 ** -7, kc.DTYPE_F16: 2.0 ** -10, F32: 2e-5}
+
+
+@pytest.mark.parametrize("dtype", [BF, kc.DTYPE_F16])
+@pytest.mark.parametrize("b,h,kv,s,d,causal,sigma", [
+    (1, 2, 1, 16, 16, True, 1.0), (1, 3, 3, 127, 64, False, 1.0), (2, 4, 2, 128, 128, True, 1.0), (1, 2, 2, 129, 80, False, 1.0),
+    (1, 2, 1, 257, 80, True, 6.0),         # peaked rows: the running maximum grows and O is rescaled
+    (1, 160, 8, 300, 64, True, 1.0),       # two query tiles a CTA, the second past the end or short
+    (2, 80, 16, 513, 128, False, 6.0), (1, 150, 150, 385, 48, True, 1.0)])
+def test_attention_of_16_bit_sequences(backend, b, h, kv, s, d, causal, sigma, dtype):
+    from helpers import attention_f64
+    q, k, v = attention_inputs(b, h, kv, s, d, dtype, s + d, sigma)
+    got = wide(run_attention(backend, q, k, v, b, h, kv, s, d, causal, dtype), dtype)
+    assert norm_max_err(got, attention_f64(wide(q, dtype), wide(k, dtype), wide(v, dtype), b, h, kv, s, d, causal, None)) <= ATTENTION_TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", [BF, kc.DTYPE_F16])
+def test_attention_of_sequences_with_values_that_are_not_finite(backend, dtype, monkeypatch):
+    # an infinite value row, a NaN key and scores of plus infinity reach exactly the rows that see them
+    b, h, kv, s, d = 1, 4, 2, 200, 64
+    q, k, v = attention_inputs(b, h, kv, s, d, dtype, 9)
+    inf, nan = (0x7f80, 0x7fc0) if dtype == BF else (0x7c00, 0x7e00)
+    v.reshape(kv, s, d)[0, 150, 3] = inf
+    k.reshape(kv, s, d)[1, 60, 5] = nan
+    v.reshape(kv, s, d)[1, 190, 7] = nan
+    got = wide(run_attention(backend, q, k, v, b, h, kv, s, d, True, dtype), dtype).reshape(h, s, d)
+    monkeypatch.setenv("HOLO_ATTN_FORCE_GENERIC", "1")
+    want = wide(run_attention(backend, q, k, v, b, h, kv, s, d, True, dtype), dtype).reshape(h, s, d)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isposinf(got), np.isposinf(want))
+    assert np.isfinite(got[:2, :150]).all() and np.isinf(got[:2, 150:, 3]).all() and np.isfinite(got[2:, :60]).all() and np.isnan(got[2:, 60:]).all()
+    fine = np.isfinite(want)
+    assert np.max(np.abs(got[fine] - want[fine])) <= ATTENTION_TOL[dtype] * np.max(np.abs(want[fine]))
