@@ -74,6 +74,13 @@ extern "C" int32_t holo_b200_ctx_create(int32_t device, holo_b200_ctx** out) {
         delete ctx;
         return holo_fail(HOLO_ERR_INIT, "backend init failed: arrival counter allocation");
     }
+    if (cudaMalloc(&ctx->split_partials, HOLO_SPLIT_PARTIAL_BYTES) != cudaSuccess) {
+        cudaFree(ctx->attn_arrivals);
+        cudaFree(ctx->dev_status);
+        cudaStreamDestroy(ctx->stream);
+        delete ctx;
+        return holo_fail(HOLO_ERR_INIT, "backend init failed: attention partials allocation");
+    }
     cudaDeviceSynchronize();   // the clears above ran on the default stream, which the context's stream does not wait for
     *out = ctx;
     return HOLO_OK;
@@ -91,6 +98,7 @@ extern "C" void holo_b200_ctx_destroy(holo_b200_ctx* ctx) {
     if (ctx->stage) cudaFree(ctx->stage);
     if (ctx->dev_status) cudaFree(ctx->dev_status);
     if (ctx->attn_arrivals) cudaFree(ctx->attn_arrivals);
+    if (ctx->split_partials) cudaFree(ctx->split_partials);
     if (ctx->causal_partials) cudaFree(ctx->causal_partials);
     if (ctx->latent_partials) cudaFree(ctx->latent_partials);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);

@@ -27,6 +27,8 @@ struct HoloMicroOp {
     uint32_t a, b, c, d;
 };
 
+constexpr uint64_t HOLO_SPLIT_PARTIAL_BYTES = 4ull << 20;
+
 struct holo_b200_ctx {
     int device = 0;
     int sm_count = 0;
@@ -45,6 +47,7 @@ struct holo_b200_ctx {
     uint32_t* dev_status = nullptr;
     float* causal_partials = nullptr;   // split-key partials of the causal attention, allocated once at a fixed size (graphs hold its address)
     float* latent_partials = nullptr;   // the same for the latent attention
+    float* split_partials = nullptr;    // split-key partials of the float-cache attention (HOLO_SPLIT_PARTIAL_BYTES, made with the context)
     uint32_t* attn_arrivals = nullptr;  // 65536 counters, zero between launches (decode attention)
     // launch every kernel with programmatic stream serialization (HOLO_PDL=0 turns it off)
     bool pdl = true;
@@ -231,6 +234,8 @@ struct HoloAttnArgs {
 int32_t holo_launch_decode_attention(holo_b200_ctx* ctx, const HoloAttnArgs& a);
 // attention_rows.cu: whole 16-bit sequences; *taken false: the shape is not one it serves
 int32_t holo_try_attention_tile(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool* taken);
+// attention_split.cu: few rows over a float cache, the keys split over the chip
+int32_t holo_try_attention_split(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool* taken);
 // gemm.cu
 int32_t holo_launch_matmul(holo_b200_ctx* ctx, const void* a, const void* b, void* out, uint32_t m, uint32_t k,
                            uint32_t n, uint8_t dtype, uint8_t fused_act, const void* residual, bool b_constant = false);

@@ -347,3 +347,33 @@ def test_attention_of_sequences_with_values_that_are_not_finite(backend, dtype, 
     assert np.isfinite(got[:2, :150]).all() and np.isinf(got[:2, 150:, 3]).all() and np.isfinite(got[2:, :60]).all() and np.isnan(got[2:, 60:]).all()
     fine = np.isfinite(want)
     assert np.max(np.abs(got[fine] - want[fine])) <= ATTENTION_TOL[dtype] * np.max(np.abs(want[fine]))
+
+
+@pytest.mark.parametrize("dtype", [F32, BF, kc.DTYPE_F16])
+@pytest.mark.parametrize("b,h,kv,past,valid,d,sigma", [
+    (1, 1, 1, 0, 0, 64, 1.0), (1, 12, 2, 100, 0, 128, 1.0), (1, 12, 2, 1531, 1531, 128, 1.0), (1, 32, 8, 3000, 2999, 128, 4.0),
+    (2, 4, 4, 77, 5, 80, 1.0), (1, 8, 1, 4097, 4000, 64, 4.0), (1, 3, 1, 700, 10 ** 9, 256, 1.0), (1, 10, 1, 2100, 2100, 200, 1.0),
+    (3, 5, 5, 999, 640, 200, 1.0), (8, 64, 16, 301, 300, 64, 1.0), (1, 7, 7, 513, 513, 16, 4.0)])
+def test_single_token_attention_over_a_float_cache(backend, b, h, kv, past, valid, d, sigma, dtype):
+    # clusters of every size and several of them per kv head, caches shorter than what they were cut for, padded row blocks
+    rng = np.random.default_rng(past + d)
+    arrs = [rng.standard_normal(n).astype(np.float32) for n in (b * h * d, b * kv * past * d, b * kv * past * d, b * kv * d, b * kv * d)]
+    arrs[0] *= sigma
+    if dtype != F32:
+        arrs = [orc.f32_to_bf16_rne(x) if dtype == BF else x.astype(np.float16).view(np.uint16) for x in arrs]
+    rc, want = orc.decode_attention_valid(*arrs, valid, b, h, kv, 1, past, 1, d, 0, dtype)
+    assert rc == 0
+    hidden = min(valid, past)          # bytes past the valid rows, NaN among them, are never read
+    for x in arrs[1:3]:
+        x.reshape(b * kv, past, d)[:, hidden:] = np.nan if dtype == F32 else 0x7fc0 if dtype == BF else 0x7e00
+    ws = hb.DeviceWorkspace(backend, 7)
+    for i, x in enumerate(arrs):
+        ws.put(i, x if x.size else np.zeros(16, x.dtype))
+    ws.put(5, np.array([valid], dtype=np.uint32))
+    ws.alloc(6, arrs[0].nbytes)
+    call = kc.KernelCall.DecodeAttentionValid(kc.DecodeAttentionValidCall(*[kc.rb(i) for i in range(7)], b, h, kv, 1, past, 1, d, 0, dtype))
+    for _ in range(2):                 # the second launch finds the counters as the first one did
+        backend.dispatch(call, ws)
+        got = ws.read(6, arrs[0].nbytes, arrs[0].dtype)
+        assert norm_max_err(wide(got, dtype), wide(want, dtype)) <= ATTENTION_TOL[dtype]
+    ws.close()
