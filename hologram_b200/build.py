@@ -14,7 +14,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libhologram_b200.so")
-SOURCES = ["api.cu", "lut.cu", "glue.cu", "attention.cu", "attention_rows.cu", "attention_split.cu", "gemm.cu", "gemm_cell.cu", "linear.cu", "causal_attention.cu", "window_attention.cu", "retention.cu", "moe.cu", "quant_gemv.cu", "tp.cu", "session.cu", "addressed.cpp", "pool.cpp", "archive.cpp", "blake3.cpp", "label.cpp"]
+SOURCES = ["api.cu", "lut.cu", "glue.cu", "attention.cu", "attention_rows.cu", "attention_f32.cu", "attention_split.cu", "gemm.cu", "gemm_cell.cu", "linear.cu", "causal_attention.cu", "window_attention.cu", "retention.cu", "moe.cu", "quant_gemv.cu", "tp.cu", "session.cu", "addressed.cpp", "pool.cpp", "archive.cpp", "blake3.cpp", "label.cpp"]
 SERVING_LIB = os.path.join(HERE, "libhologram_b200_serving.so")
 SERVING_SOURCES = ["api.cu", "glue.cu", "linear.cu", "causal_attention.cu", "window_attention.cu", "retention.cu", "moe.cu", "session.cu", "addressed.cpp", "pool.cpp", "archive.cpp", "blake3.cpp", "label.cpp",
                    "absent_families.cpp"]

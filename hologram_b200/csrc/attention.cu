@@ -850,6 +850,7 @@ int32_t holo_launch_decode_attention(holo_b200_ctx* ctx, const HoloAttnArgs& a) 
     if (!getenv("HOLO_ATTN_FORCE_GENERIC")) {
         bool taken = false;
         HOLO_TRY(holo_try_attention_tile(ctx, a, &taken));
+        if (!taken) HOLO_TRY(holo_try_attention_f32(ctx, a, &taken));
         if (!taken) HOLO_TRY(holo_try_attention_split(ctx, a, &taken));
         if (taken) return HOLO_OK;
     }

@@ -234,6 +234,8 @@ struct HoloAttnArgs {
 int32_t holo_launch_decode_attention(holo_b200_ctx* ctx, const HoloAttnArgs& a);
 // attention_rows.cu: whole 16-bit sequences; *taken false: the shape is not one it serves
 int32_t holo_try_attention_tile(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool* taken);
+// attention_f32.cu: many f32 rows, with or without a cache before them
+int32_t holo_try_attention_f32(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool* taken);
 // attention_split.cu: few rows over a float cache, the keys split over the chip
 int32_t holo_try_attention_split(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool* taken);
 // gemm.cu

@@ -331,12 +331,12 @@ def test_attention_of_16_bit_sequences(backend, b, h, kv, s, d, causal, sigma, d
     assert norm_max_err(got, attention_f64(wide(q, dtype), wide(k, dtype), wide(v, dtype), b, h, kv, s, d, causal, None)) <= ATTENTION_TOL[dtype]
 
 
-@pytest.mark.parametrize("dtype", [BF, kc.DTYPE_F16])
+@pytest.mark.parametrize("dtype", [BF, kc.DTYPE_F16, F32])
 def test_attention_of_sequences_with_values_that_are_not_finite(backend, dtype, monkeypatch):
     # an infinite value row, a NaN key and scores of plus infinity reach exactly the rows that see them
     b, h, kv, s, d = 1, 4, 2, 200, 64
     q, k, v = attention_inputs(b, h, kv, s, d, dtype, 9)
-    inf, nan = (0x7f80, 0x7fc0) if dtype == BF else (0x7c00, 0x7e00)
+    inf, nan = (0x7f80, 0x7fc0) if dtype == BF else (0x7c00, 0x7e00) if dtype != F32 else (np.inf, np.nan)
     v.reshape(kv, s, d)[0, 150, 3] = inf
     k.reshape(kv, s, d)[1, 60, 5] = nan
     v.reshape(kv, s, d)[1, 190, 7] = nan
@@ -376,4 +376,33 @@ def test_single_token_attention_over_a_float_cache(backend, b, h, kv, past, vali
         backend.dispatch(call, ws)
         got = ws.read(6, arrs[0].nbytes, arrs[0].dtype)
         assert norm_max_err(wide(got, dtype), wide(want, dtype)) <= ATTENTION_TOL[dtype]
+    ws.close()
+
+
+@pytest.mark.parametrize("b,h,kv,s,d,causal,sigma", [
+    (1, 1, 1, 2, 4, True, 1.0), (1, 4, 2, 63, 64, True, 1.0), (2, 3, 3, 65, 64, False, 6.0), (1, 12, 12, 381, 64, False, 1.0), (1, 60, 20, 200, 64, True, 1.0),
+    (1, 4, 1, 129, 80, True, 6.0), (1, 2, 2, 100, 96, False, 1.0), (1, 40, 8, 257, 128, True, 1.0), (1, 3, 3, 320, 112, False, 6.0), (1, 2, 1, 70, 20, True, 1.0)])
+def test_attention_of_f32_sequences(backend, b, h, kv, s, d, causal, sigma):
+    from helpers import attention_f64
+    q, k, v = attention_inputs(b, h, kv, s, d, F32, s + d, sigma)
+    got = run_attention(backend, q, k, v, b, h, kv, s, d, causal, F32)
+    assert norm_max_err(got, attention_f64(q, k, v, b, h, kv, s, d, causal, None)) <= ATTENTION_TOL[F32]
+
+
+@pytest.mark.parametrize("past,valid,m,d", [(100, 100, 5, 64), (70, 0, 33, 128), (64, 64, 64, 64), (300, 211, 130, 96)])
+def test_chunk_of_f32_rows_after_a_cache(backend, past, valid, m, d):
+    b, h, kv = 2, 6, 2
+    rng = np.random.default_rng(past + m)
+    arrs = [rng.standard_normal(n).astype(np.float32) for n in (b * h * m * d, b * kv * past * d, b * kv * past * d, b * kv * m * d, b * kv * m * d)]
+    rc, want = orc.decode_attention_valid(*arrs, valid, b, h, kv, m, past, m, d, 0, F32)
+    assert rc == 0
+    for x in arrs[1:3]:
+        x.reshape(b * kv, past, d)[:, valid:] = np.nan        # never read
+    ws = hb.DeviceWorkspace(backend, 7)
+    for i, x in enumerate(arrs):
+        ws.put(i, x)
+    ws.put(5, np.array([valid], dtype=np.uint32))
+    ws.alloc(6, arrs[0].nbytes)
+    backend.dispatch(kc.KernelCall.DecodeAttentionValid(kc.DecodeAttentionValidCall(*[kc.rb(i) for i in range(7)], b, h, kv, m, past, m, d, 0, F32)), ws)
+    assert norm_max_err(ws.read(6, arrs[0].nbytes, np.float32), want) <= ATTENTION_TOL[F32]
     ws.close()
