@@ -9,15 +9,17 @@
 //   * Groups of lanes, warps and CTAs each keep a (maximum, sum, context) triple; warps merge through shared memory, the CTAs of
 //     a cluster through distributed shared memory (each CTA a slice of the cells), clusters through a buffer that the last one
 //     to count in reads. Nobody waits for another cluster.
-// Measured, us (one CTA per query row with a warp per key, before, in brackets): f32, 12 heads over 2, dim 128, 8192 keys 19.1 [2471];
-// f32, 8 sequences, 32 over 8, 8192 keys 87 = 6.1 TB/s; bf16 the same 62 = 4.4 TB/s (two warps per scheduler, a turn's chain of
-// product, halving, division and exponential); bf16, 8 sequences of 16 heads, dim 64 46 = 5.8 TB/s; 100 keys 5.
+// Measured, us (one CTA per query row with a warp per key, before, in brackets): f32, 12 heads over 2, dim 128, 8192 keys 14.4 [2471];
+// f32, 8 sequences, 32 over 8, 8192 keys 88 = 6.1 TB/s; bf16 the same 59 = 4.5 TB/s (two warps per scheduler, a turn's chain of
+// product, halving, division and exponential); bf16, 8 sequences of 16 heads, dim 64 47 = 5.7 TB/s; 100 keys 5.3. The first figure
+// was 18.8 with a rescaling at every new maximum and the parts' statistics and cells requested one after the other.
 #include "common.h"
 #include "numerics.cuh"
 
 namespace {
 
 constexpr int WARPS = 8;
+constexpr float GROWTH = 8.0f;
 constexpr uint32_t MAX_CLUSTER = 8, MAX_CLUSTERS = 16;            // CTAs of a cluster; clusters that share a kv head
 constexpr uint32_t SLOT_CELLS = 8 * 256, SLOT_FLOATS = SLOT_CELLS + MAX_CLUSTER * 8 * 2;   // cells, then (maximum, sum) per row from each CTA of the cluster
 constexpr uint32_t SLOTS = HOLO_SPLIT_PARTIAL_BYTES / (SLOT_FLOATS * 4);
@@ -223,7 +225,8 @@ attention_split_kernel(const __grid_constant__ Params p) {
             }
         }
         const float s = key_of(turn, mine / RB) < key1 ? __fdiv_rn(part[0], a.scale_div) : -INFINITY;
-        if (__any_sync(0xffffffffu, s > top)) {
+        // a row's context is rescaled only when its maximum has grown by more than e^GROWTH: weights stay far inside f32's range
+        if (__any_sync(0xffffffffu, s > top + GROWTH)) {
             float next = fmaxf(top, s);
 #pragma unroll
             for (int step = LK / 2; step > LK / 2 / KU; step /= 2) next = fmaxf(next, __shfl_xor_sync(0xffffffffu, next, step));
@@ -302,16 +305,20 @@ attention_split_kernel(const __grid_constant__ Params p) {
     __syncthreads();
     // One thread per row works out the parts' weights, then all threads add four cells at a time.
     const uint32_t vecs = rows * a.d / 4, tid = threadIdx.x;
-    auto weigh = [&](uint32_t n, auto ml) {     // ml(part) -> (maximum, sum) of row `tid`
+    auto weigh = [&](uint32_t n, auto ml) {     // ml(part) -> (maximum, sum) of row `tid`, requested all at once
+        float2 v[MAX_CLUSTERS];
         float common = -INFINITY, total = 0.0f;
-#pragma unroll 8
-        for (uint32_t c = 0; c < n; ++c) common = fmaxf(common, ml(c).x);
-#pragma unroll 8
-        for (uint32_t c = 0; c < n; ++c) {
-            const float2 v = ml(c);
-            const float f = share(v.x, common);
-            s_f[c][tid] = f;
-            total = fmaf(f, v.y, total);
+#pragma unroll
+        for (uint32_t c = 0; c < MAX_CLUSTERS; ++c) v[c] = c < n ? ml(c) : make_float2(-INFINITY, 0.0f);
+#pragma unroll
+        for (uint32_t c = 0; c < MAX_CLUSTERS; ++c) common = fmaxf(common, v[c].x);
+#pragma unroll
+        for (uint32_t c = 0; c < MAX_CLUSTERS; ++c) {
+            if (c < n) {
+                const float f = share(v[c].x, common);
+                s_f[c][tid] = f;
+                total = fmaf(f, v[c].y, total);
+            }
         }
         return make_float2(common, total);
     };
@@ -366,21 +373,33 @@ attention_split_kernel(const __grid_constant__ Params p) {
     if (p.cluster > 1) cluster_sync();     // the others have read this CTA's cells
     if (used == 1) return;
     // ---- clusters: the last one to count in adds them up, slice by slice ----
-    __threadfence();
     __syncthreads();
-    if (tid == 0) s_last = atomicAdd(p.arrivals + blockIdx.y * p.cluster + rank, 1u) == used - 1 ? 1u : 0u;
+    if (tid == 0) {     // the barrier orders the others' stores before this fence
+        __threadfence();
+        s_last = atomicAdd(p.arrivals + blockIdx.y * p.cluster + rank, 1u) == used - 1 ? 1u : 0u;
+        __threadfence();
+    }
     __syncthreads();
     if (!s_last) return;
-    __threadfence();
     if (tid == 0) p.arrivals[blockIdx.y * p.cluster + rank] = 0;
     const float* all = p.partials + (uint64_t)blockIdx.y * p.clusters * SLOT_FLOATS;
+    // a thread's first cells are requested along with the weights
+    float4 v[MAX_CLUSTERS];
+    auto fetch = [&](uint32_t i) {
+#pragma unroll
+        for (uint32_t c = 0; c < MAX_CLUSTERS; ++c)
+            v[c] = c < used && i < end ? __ldcg(reinterpret_cast<const float4*>(all + (uint64_t)c * SLOT_FLOATS) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    fetch(begin + tid);
     if (tid < RB) s_sum[tid] = weigh(used, [&](uint32_t c) { return __ldcg(reinterpret_cast<const float2*>(all + (uint64_t)c * SLOT_FLOATS + SLOT_CELLS) + rank * 8 + tid); }).y;
     __syncthreads();
     for (uint32_t i = begin + tid; i < end; i += WARPS * 32) {
+        if (i != begin + tid) fetch(i);
         const uint32_t r = 4 * i / a.d;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-        for (uint32_t c = 0; c < used; ++c) add_scaled(acc, s_f[c][r], __ldcg(reinterpret_cast<const float4*>(all + (uint64_t)c * SLOT_FLOATS) + i));
+#pragma unroll
+        for (uint32_t c = 0; c < MAX_CLUSTERS; ++c)
+            if (c < used) add_scaled(acc, s_f[c][r], v[c]);
         finish(i, s_sum[r], acc);
     }
 }
