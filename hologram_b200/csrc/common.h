@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <mutex>
 #include <vector>
 
 #include "../../include/hologram_b200.h"
@@ -28,6 +29,7 @@ struct HoloMicroOp {
 };
 
 constexpr uint64_t HOLO_SPLIT_PARTIAL_BYTES = 4ull << 20;
+constexpr uint64_t HOLO_HOST_STAGE_BYTES = 1ull << 20;
 
 struct holo_b200_ctx {
     int device = 0;
@@ -43,6 +45,9 @@ struct holo_b200_ctx {
     // device staging arena used by the host-workspace dispatch form
     void* stage = nullptr;
     uint64_t stage_bytes = 0;
+    // pinned memory that downloads and the error word pass through, one at a time
+    uint8_t* host_stage = nullptr;
+    std::mutex host_mutex;
     // device-side error word (bounded waits record where they gave up)
     uint32_t* dev_status = nullptr;
     float* causal_partials = nullptr;   // split-key partials of the causal attention, allocated once at a fixed size (graphs hold its address)
