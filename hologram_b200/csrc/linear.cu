@@ -93,9 +93,12 @@ rms_norm_multi_kernel(const float* __restrict__ x, const float* __restrict__ gam
     const uint32_t nvec = feature >> 2;
     holo_pdl_wait();
     const float* row = x + (uint64_t)blockIdx.x * feature;
-    float4 v[NORM_VECS];
+    float4 v[NORM_VECS], first[2];      // the scales of a thread's first vector are requested along with the row, not after its sum
     float acc = 0.0f;
     if (VEC) {
+        const bool one = tid < nvec;
+        first[0] = one ? reinterpret_cast<const float4*>(gamma0)[tid] : make_float4(0.f, 0.f, 0.f, 0.f);
+        first[1] = one && gamma1 ? reinterpret_cast<const float4*>(gamma1)[tid] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < NORM_VECS; ++i) {
             const uint32_t j = tid + i * nt;
@@ -122,7 +125,7 @@ rms_norm_multi_kernel(const float* __restrict__ x, const float* __restrict__ gam
             for (int i = 0; i < NORM_VECS; ++i) {
                 const uint32_t j = tid + i * nt;
                 if (j < nvec) {
-                    const float4 g = reinterpret_cast<const float4*>(gm)[j];
+                    const float4 g = i == 0 ? (w ? first[1] : first[0]) : reinterpret_cast<const float4*>(gm)[j];
                     store_norm4(out, off + 4 * j, make_float4(v[i].x * inv * g.x, v[i].y * inv * g.y, v[i].z * inv * g.z, v[i].w * inv * g.w));
                 }
             }
@@ -295,11 +298,16 @@ rms_norm_parts_kernel(const HoloNormPartsArgs a) {
         else return make_float4(x[j], 0.f, 0.f, 0.f);
     };
     auto square = [](const float4& v, float acc) { return fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, acc)))); };
-    float4 held[PARTS_HELD];
+    auto weight_of = [&](uint32_t j) {
+        if constexpr (VEC) return p.weight ? reinterpret_cast<const float4*>(p.weight)[j] : make_float4(1.f, 1.f, 1.f, 1.f);
+        else return make_float4(p.weight ? p.weight[j] : 1.0f, 0.f, 0.f, 0.f);
+    };
+    float4 held[PARTS_HELD], weight[PARTS_HELD];       // the weights are requested along with the row, not after its sum
 #pragma unroll
     for (int i = 0; i < PARTS_HELD; ++i) {
         const uint32_t j = tid + PARTS_THREADS * i;
         held[i] = j < nvec ? fetch(j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        weight[i] = j < nvec ? weight_of(j) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     uint64_t orow = row;
     if (p.ring) {
@@ -321,20 +329,19 @@ rms_norm_parts_kernel(const HoloNormPartsArgs a) {
         inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(acc, (float)p.width), a.eps)));
     }
     T* out = (T*)p.out + orow * p.ld;
-    auto put = [&](uint32_t j, const float4& v) {
+    auto put = [&](uint32_t j, const float4& v, const float4& w) {
         if constexpr (VEC) {
-            const float4 w = p.weight ? reinterpret_cast<const float4*>(p.weight)[j] : make_float4(1.f, 1.f, 1.f, 1.f);
             store_norm4(out, 4 * j, make_float4(v.x * inv * w.x, v.y * inv * w.y, v.z * inv * w.z, v.w * inv * w.w));
         } else {
-            store_norm(out, j, v.x * inv * (p.weight ? p.weight[j] : 1.0f));
+            store_norm(out, j, v.x * inv * w.x);
         }
     };
 #pragma unroll
     for (int i = 0; i < PARTS_HELD; ++i) {
         const uint32_t j = tid + PARTS_THREADS * i;
-        if (j < nvec) put(j, held[i]);
+        if (j < nvec) put(j, held[i], weight[i]);
     }
-    for (uint32_t j = tid + PARTS_THREADS * PARTS_HELD; j < nvec; j += PARTS_THREADS) put(j, fetch(j));
+    for (uint32_t j = tid + PARTS_THREADS * PARTS_HELD; j < nvec; j += PARTS_THREADS) put(j, fetch(j), weight_of(j));
     for (uint32_t j = p.width + tid; j < p.out_width; j += PARTS_THREADS) store_norm(out, j, 0.0f);
 }
 

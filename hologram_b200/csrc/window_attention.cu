@@ -321,7 +321,7 @@ latent_attention_kernel(const LatentParams p) {
 }
 
 // One CTA per (pair, 128 value columns). At most MERGE_SPLITS shares.
-constexpr uint32_t MERGE_SPLITS = 256;
+constexpr uint32_t MERGE_SPLITS = 256, MERGE_EARLY = 32;
 template <int KT>
 __global__ void __launch_bounds__(128)
 latent_merge_kernel(const LatentParams p) {
@@ -330,17 +330,26 @@ latent_merge_kernel(const LatentParams p) {
     const uint32_t pair = blockIdx.x, tile = pair >> 4, row = pair / a.heads, head = pair % a.heads, tid = threadIdx.x, c = blockIdx.y * 128 + tid;
     holo_pdl_trigger();
     holo_pdl_wait();
-    const LatentRange range = latent_range(a, tile, *a.pos);
-    const uint32_t used = min(p.splits, (range.hi - range.lo + KT) / KT), ml = a.vdim + 2;
-    if (used < 2) return;
+    // everything is requested at once: the position, and of every share that may be in use its statistics and (the first ones') values
+    const uint32_t ml = a.vdim + 2;
     const float* part = p.partials + (uint64_t)tile * p.splits * 16 * ml + (pair & 15u) * ml;
-    const float sink = a.sink ? a.sink[head] * LOG2E : -INFINITY;
     float2 mine[MERGE_SPLITS / 128];
-    float top = sink;
+    float early[MERGE_EARLY];
 #pragma unroll
     for (uint32_t i = 0; i < MERGE_SPLITS / 128; ++i) {
         const uint32_t share = tid + 128 * i;
-        mine[i] = share < used ? *reinterpret_cast<const float2*>(part + (uint64_t)share * 16 * ml + a.vdim) : make_float2(-INFINITY, 0.0f);
+        mine[i] = share < p.splits ? *reinterpret_cast<const float2*>(part + (uint64_t)share * 16 * ml + a.vdim) : make_float2(-INFINITY, 0.0f);
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < MERGE_EARLY; ++i) early[i] = c < a.vdim && i < p.splits ? part[(uint64_t)i * 16 * ml + c] : 0.0f;
+    const LatentRange range = latent_range(a, tile, *a.pos);
+    const uint32_t used = min(p.splits, (range.hi - range.lo + KT) / KT);
+    if (used < 2) return;
+    const float sink = a.sink ? a.sink[head] * LOG2E : -INFINITY;
+    float top = sink;
+#pragma unroll
+    for (uint32_t i = 0; i < MERGE_SPLITS / 128; ++i) {
+        if (tid + 128 * i >= used) mine[i] = make_float2(-INFINITY, 0.0f);
         top = fmaxf(top, mine[i].x);
     }
     for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
@@ -361,8 +370,11 @@ latent_merge_kernel(const LatentParams p) {
     if (c >= a.vdim) return;
     denom = (s_red[4] + s_red[5]) + (s_red[6] + s_red[7]) + exp2f(sink - top);
     float acc = 0.0f;
+#pragma unroll
+    for (uint32_t i = 0; i < MERGE_EARLY; ++i)
+        if (i < used) acc = fmaf(early[i], s_factor[i], acc);
 #pragma unroll 16
-    for (uint32_t i = 0; i < used; ++i) acc = fmaf(part[(uint64_t)i * 16 * ml + c], s_factor[i], acc);
+    for (uint32_t i = MERGE_EARLY; i < used; ++i) acc = fmaf(part[(uint64_t)i * 16 * ml + c], s_factor[i], acc);
     ((__nv_bfloat16*)a.out)[(uint64_t)row * a.ld + (uint64_t)head * a.vdim + c] = __float2bfloat16_rn(acc / denom);
 }
 
