@@ -9,6 +9,9 @@
 //   * Groups of lanes, warps and CTAs each keep a (maximum, sum, context) triple; warps merge through shared memory, the CTAs of
 //     a cluster through distributed shared memory (each CTA a slice of the cells), clusters through a buffer that the last one
 //     to count in reads. Nobody waits for another cluster.
+//   * That buffer and its counters are the context's, and launches on its stream take turns with them. A graph that a caller
+//     records may be replayed beside another one, on any stream: such a launch keeps to one cluster per kv head and touches
+//     nothing but its operands.
 // Measured, us (one CTA per query row with a warp per key, before, in brackets): f32, 12 heads over 2, dim 128, 8192 keys 14.4 [2471];
 // f32, 8 sequences, 32 over 8, 8192 keys 88 = 6.1 TB/s; bf16 the same 59 = 4.5 TB/s (two warps per scheduler, a turn's chain of
 // product, halving, division and exponential); bf16, 8 sequences of 16 heads, dim 64 47 = 5.7 TB/s; 100 keys 5.3. The first figure
@@ -29,6 +32,7 @@ struct Params {
     float* partials;
     uint32_t* arrivals;
     uint32_t rows, rowblocks, clusters, cluster;   // query rows of a kv head; clusters per (kv head, row block), CTAs per cluster
+    uint32_t max_clusters;                         // 1 where the partials may not be used
 };
 
 __device__ __forceinline__ uint64_t pair(float lo, float hi) {
@@ -432,7 +436,7 @@ int32_t launch(holo_b200_ctx* ctx, Params p, uint32_t items) {
     const uint64_t keys = (uint64_t)p.a.past + p.a.nnew;
     uint64_t best = ~0ull;
     for (uint32_t i = 0; i < 4; ++i)
-        for (uint32_t n = 1; n <= MAX_CLUSTERS; ++n) {
+        for (uint32_t n = 1; n <= p.max_clusters; ++n) {
             const uint64_t ctas = (uint64_t)n << i, waves = ((uint64_t)items * n + resident[i] - 1) / resident[i];
             if (ctas > 1 && (ctas * WARPS * S::KEYS > keys || (n > 1 && (uint64_t)items * n > SLOTS))) break;
             const uint64_t cost = waves * ((keys + ctas - 1) / ctas + 64 + (i ? 64 : 0) + (n > 1 ? 64 + 4 * n : 0));
@@ -468,7 +472,9 @@ int32_t holo_try_attention_split(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool
     if (a.d % vec != 0 || a.d > 256 || rows > 64 || keys > 0x7fffffffull) return HOLO_OK;
     const uintptr_t cache = a.past ? (uintptr_t)a.k_past | (uintptr_t)a.v_past : 0;
     if (((cache | (uintptr_t)a.q | (uintptr_t)a.k_new | (uintptr_t)a.v_new) & 15u) != 0) return HOLO_OK;
-    Params p = {a, ctx->split_partials, ctx->attn_arrivals, (uint32_t)rows, 1, 1, 1};
+    cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
+    if (!ctx->session_capture) HOLO_CUDA(cudaStreamIsCapturing(ctx->stream, &recording));
+    Params p = {a, ctx->split_partials, ctx->attn_arrivals, (uint32_t)rows, 1, 1, 1, recording == cudaStreamCaptureStatusNone ? MAX_CLUSTERS : 1};
     const uint64_t planes = (uint64_t)a.b * a.hkv;
     if (a.dtype == HOLO_DTYPE_F32) return launch_sized<HOLO_DTYPE_F32>(ctx, p, planes, taken);
     return a.dtype == HOLO_DTYPE_F16 ? launch_sized<HOLO_DTYPE_F16>(ctx, p, planes, taken) : launch_sized<HOLO_DTYPE_BF16>(ctx, p, planes, taken);

@@ -53,6 +53,7 @@ struct holo_b200_ctx {
     float* causal_partials = nullptr;   // split-key partials of the causal attention, allocated once at a fixed size (graphs hold its address)
     float* latent_partials = nullptr;   // the same for the latent attention
     float* split_partials = nullptr;    // split-key partials of the float-cache attention (HOLO_SPLIT_PARTIAL_BYTES, made with the context)
+    bool session_capture = false;       // the stream is recording a session's own walk: its replays are ordered on this stream too
     uint32_t* attn_arrivals = nullptr;  // 65536 counters, zero between launches (decode attention)
     // launch every kernel with programmatic stream serialization (HOLO_PDL=0 turns it off)
     bool pdl = true;

@@ -1034,7 +1034,9 @@ extern "C" int32_t holo_b200_session_capture(holo_b200_session* s) {
     }
     HOLO_CUDA(cudaStreamSynchronize(s->ctx->stream));
     HOLO_CUDA(cudaStreamBeginCapture(s->ctx->stream, cudaStreamCaptureModeThreadLocal));
+    s->ctx->session_capture = true;
     int32_t rc = run_calls(s);
+    s->ctx->session_capture = false;
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(s->ctx->stream, &g);
     if (rc != HOLO_OK) {

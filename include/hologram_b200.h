@@ -630,7 +630,11 @@ void holo_b200_ctx_destroy(holo_b200_ctx* ctx);
 /* The CUDA stream (cudaStream_t) every dispatch is ordered on. */
 void* holo_b200_ctx_stream(holo_b200_ctx* ctx);
 /* Order every later dispatch on a caller-owned stream instead (e.g. the host framework's
- * current stream, so its events bracket these kernels). */
+ * current stream, so its events bracket these kernels). Calls recorded there (stream capture)
+ * may be replayed on any stream; graphs recorded from one context must not run side by side
+ * where they hold calls that work in the context's buffers (attention over an int8 cache, causal
+ * and latent attention of few rows, products with a [k, n] quantized weight). Attention over a
+ * float cache is recorded without them and may. */
 int32_t holo_b200_ctx_set_stream(holo_b200_ctx* ctx, void* cuda_stream);
 /* Wait for the stream; also reports device-side failures recorded since the last check
  * (an out-of-range Gather index, a bounded wait that gave up). */

@@ -379,6 +379,52 @@ def test_single_token_attention_over_a_float_cache(backend, b, h, kv, past, vali
     ws.close()
 
 
+@pytest.mark.parametrize("dtype", [F32, BF])
+def test_recorded_calls_of_one_context_share_nothing(dtype):
+    # two graphs recorded from one context, replayed side by side on two streams: each gives its own call's result every time
+    import torch
+    b, h, kv, past, d = 1, 12, 2, 4000, 128
+    be, kind = hb.B200Backend(0), torch.float32 if dtype == F32 else torch.bfloat16
+    stream = torch.cuda.Stream()
+    be.set_stream(stream.cuda_stream)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    graphs, outs, wants, kept = [], [], [], []
+    for _ in range(2):
+        x = [torch.randn(n, generator=g, device="cuda").to(kind) for n in (b * h * d, b * kv * past * d, b * kv * past * d, b * kv * d, b * kv * d)]
+        x += [torch.tensor([past], dtype=torch.int32, device="cuda"), torch.empty(b * h * d, device="cuda", dtype=kind)]
+        torch.cuda.synchronize()
+        ws = hb.DeviceWorkspace(be, 7)
+        for i, t in enumerate(x):
+            ws.bind(i, t.data_ptr(), t.numel() * t.element_size())
+        call = kc.KernelCall.DecodeAttentionValid(kc.DecodeAttentionValidCall(*[kc.rb(i) for i in range(7)], b, h, kv, 1, past, 1, d, 0, dtype))
+        be.dispatch(call, ws)
+        be.synchronize()
+        wants.append(x[6].double().clone())
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            be.dispatch(call, ws)
+        graphs.append(graph)
+        outs.append(x[6])
+        kept.append((x, ws))
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in graphs], [[], []]
+    for _ in range(50):
+        for i, graph in enumerate(graphs):
+            with torch.cuda.stream(streams[i]):
+                outs[i].fill_(float("nan"))
+                graph.replay()
+                got[i].append(outs[i].clone())
+    torch.cuda.synchronize()
+    tol = 2.0 ** -7 if dtype == BF else 2e-5      # ATTENTION_TOL: the recorded call adds up in another order
+    for want, results in zip(wants, got):
+        for r in results:
+            assert (r.double() - want).abs().max() <= tol * want.abs().max()
+    for x, ws in kept:
+        ws.close()
+    del graphs
+    be.close()
+
+
 @pytest.mark.parametrize("b,h,kv,s,d,causal,sigma", [
     (1, 1, 1, 2, 4, True, 1.0), (1, 4, 2, 63, 64, True, 1.0), (2, 3, 3, 65, 64, False, 6.0), (1, 12, 12, 381, 64, False, 1.0), (1, 60, 20, 200, 64, True, 1.0),
     (1, 4, 1, 129, 80, True, 6.0), (1, 2, 2, 100, 96, False, 1.0), (1, 40, 8, 257, 128, True, 1.0), (1, 3, 3, 320, 112, False, 6.0), (1, 2, 1, 70, 20, True, 1.0)])
