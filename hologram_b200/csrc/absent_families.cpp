@@ -11,6 +11,7 @@ int32_t absent(const char* what) {
 int32_t holo_lut_table(holo_b200_ctx*, uint8_t, uint8_t, const uint16_t**) { return absent("LUT activation"); }
 int32_t holo_launch_lut(holo_b200_ctx*, const uint16_t*, const uint16_t*, uint16_t*, uint64_t) { return absent("LUT activation"); }
 int32_t holo_launch_decode_attention(holo_b200_ctx*, const HoloAttnArgs&) { return absent("decode attention"); }
+void holo_split_partials_create(holo_b200_ctx*) {}
 int32_t holo_launch_matmul(holo_b200_ctx*, const void*, const void*, void*, uint32_t, uint32_t, uint32_t, uint8_t, uint8_t, const void*, bool) { return absent("matmul"); }
 int32_t holo_launch_matmul_add_activation(holo_b200_ctx*, const void*, const void*, void*, uint32_t, uint32_t, uint32_t, uint8_t, uint8_t, const void*) { return absent("matmul"); }
 int32_t holo_launch_matmul_multi(holo_b200_ctx*, const void*, const void*, uint32_t, uint32_t, uint32_t, uint8_t, const HoloMatmulSeg*, uint32_t) { return absent("matmul"); }

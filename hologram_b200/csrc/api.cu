@@ -74,13 +74,7 @@ extern "C" int32_t holo_b200_ctx_create(int32_t device, holo_b200_ctx** out) {
         delete ctx;
         return holo_fail(HOLO_ERR_INIT, "backend init failed: arrival counter allocation");
     }
-    if (cudaMalloc(&ctx->split_partials, HOLO_SPLIT_PARTIAL_BYTES) != cudaSuccess) {
-        cudaFree(ctx->attn_arrivals);
-        cudaFree(ctx->dev_status);
-        cudaStreamDestroy(ctx->stream);
-        delete ctx;
-        return holo_fail(HOLO_ERR_INIT, "backend init failed: attention partials allocation");
-    }
+    holo_split_partials_create(ctx);
     // without it downloads go straight to the caller's memory
     if (cudaHostAlloc((void**)&ctx->host_stage, HOLO_HOST_STAGE_BYTES + 64, cudaHostAllocDefault) != cudaSuccess) {
         ctx->host_stage = nullptr;

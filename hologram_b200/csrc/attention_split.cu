@@ -11,7 +11,7 @@
 //     to count in reads. Nobody waits for another cluster.
 //   * That buffer and its counters are the context's, and launches on its stream take turns with them. A graph that a caller
 //     records may be replayed beside another one, on any stream: such a launch keeps to one cluster per kv head and touches
-//     nothing but its operands.
+//     nothing but its operands (f32, 12 heads over 2, 8192 keys then 39 us instead of 14.6). So does a context without the buffer.
 // Measured, us (one CTA per query row with a warp per key, before, in brackets): f32, 12 heads over 2, dim 128, 8192 keys 14.4 [2471];
 // f32, 8 sequences, 32 over 8, 8192 keys 88 = 6.1 TB/s; bf16 the same 59 = 4.5 TB/s (two warps per scheduler, a turn's chain of
 // product, halving, division and exponential); bf16, 8 sequences of 16 heads, dim 64 47 = 5.7 TB/s; 100 keys 5.3. The first figure
@@ -463,6 +463,12 @@ int32_t launch_sized(holo_b200_ctx* ctx, Params p, uint64_t planes, bool* taken)
 
 }  // namespace
 
+void holo_split_partials_create(holo_b200_ctx* ctx) {
+    if (cudaMalloc(&ctx->split_partials, HOLO_SPLIT_PARTIAL_BYTES) == cudaSuccess) return;
+    ctx->split_partials = nullptr;
+    cudaGetLastError();
+}
+
 int32_t holo_try_attention_split(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool* taken) {
     *taken = false;
     // every row must see the same keys: a weight of zero times an infinite value would not be zero
@@ -474,7 +480,8 @@ int32_t holo_try_attention_split(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool
     if (((cache | (uintptr_t)a.q | (uintptr_t)a.k_new | (uintptr_t)a.v_new) & 15u) != 0) return HOLO_OK;
     cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
     if (!ctx->session_capture) HOLO_CUDA(cudaStreamIsCapturing(ctx->stream, &recording));
-    Params p = {a, ctx->split_partials, ctx->attn_arrivals, (uint32_t)rows, 1, 1, 1, recording == cudaStreamCaptureStatusNone ? MAX_CLUSTERS : 1};
+    const bool shared = ctx->split_partials && recording == cudaStreamCaptureStatusNone;
+    Params p = {a, ctx->split_partials, ctx->attn_arrivals, (uint32_t)rows, 1, 1, 1, shared ? MAX_CLUSTERS : 1};
     const uint64_t planes = (uint64_t)a.b * a.hkv;
     if (a.dtype == HOLO_DTYPE_F32) return launch_sized<HOLO_DTYPE_F32>(ctx, p, planes, taken);
     return a.dtype == HOLO_DTYPE_F16 ? launch_sized<HOLO_DTYPE_F16>(ctx, p, planes, taken) : launch_sized<HOLO_DTYPE_BF16>(ctx, p, planes, taken);

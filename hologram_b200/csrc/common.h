@@ -52,7 +52,7 @@ struct holo_b200_ctx {
     uint32_t* dev_status = nullptr;
     float* causal_partials = nullptr;   // split-key partials of the causal attention, allocated once at a fixed size (graphs hold its address)
     float* latent_partials = nullptr;   // the same for the latent attention
-    float* split_partials = nullptr;    // split-key partials of the float-cache attention (HOLO_SPLIT_PARTIAL_BYTES, made with the context)
+    float* split_partials = nullptr;    // split-key partials of the float-cache attention (HOLO_SPLIT_PARTIAL_BYTES, made with the context) or null
     bool session_capture = false;       // the stream is recording a session's own walk: its replays are ordered on this stream too
     uint32_t* attn_arrivals = nullptr;  // 65536 counters, zero between launches (decode attention)
     // launch every kernel with programmatic stream serialization (HOLO_PDL=0 turns it off)
@@ -244,6 +244,7 @@ int32_t holo_try_attention_tile(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool*
 int32_t holo_try_attention_f32(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool* taken);
 // attention_split.cu: few rows over a float cache, the keys split over the chip
 int32_t holo_try_attention_split(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool* taken);
+void holo_split_partials_create(holo_b200_ctx* ctx);   // with the context: a launch can allocate nothing. Where it fails, launches do without
 // gemm.cu
 int32_t holo_launch_matmul(holo_b200_ctx* ctx, const void* a, const void* b, void* out, uint32_t m, uint32_t k,
                            uint32_t n, uint8_t dtype, uint8_t fused_act, const void* residual, bool b_constant = false);
