@@ -45,7 +45,7 @@ struct holo_b200_ctx {
     // device staging arena used by the host-workspace dispatch form
     void* stage = nullptr;
     uint64_t stage_bytes = 0;
-    // pinned memory that downloads and the error word pass through, one at a time
+    // pinned memory that downloads to pageable memory and the error word pass through; whoever finds the mutex taken does without
     uint8_t* host_stage = nullptr;
     std::mutex host_mutex;
     // device-side error word (bounded waits record where they gave up)
