@@ -346,14 +346,22 @@ rms_norm_parts_kernel(const HoloNormPartsArgs a) {
 }
 
 // A CTA takes HEAD_COLS columns of one head for up to R rows; its threads split k and add up through shared memory.
-constexpr int HEAD_THREADS = 256, HEAD_BATCH = 8;
+constexpr int HEAD_THREADS = 256;
 template <typename T> struct HeadVec;
 template <> struct HeadVec<float> { static constexpr int N = 4; };
 template <> struct HeadVec<__nv_bfloat16> { static constexpr int N = 8; };
 template <typename T>
-__device__ __forceinline__ void load_part(const T* src, uint32_t left, float (&v)[HeadVec<T>::N]) {
+__device__ __forceinline__ void load_vec(const T* src, bool vec, uint32_t left, float (&v)[HeadVec<T>::N]) {
+    constexpr int N = HeadVec<T>::N;
+    if (vec) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(src);
+        const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-    for (int i = 0; i < HeadVec<T>::N; ++i) v[i] = (uint32_t)i < left ? (float)src[i] : 0.0f;
+        for (int i = 0; i < N; ++i) v[i] = (float)e[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i] = (uint32_t)i < left ? (float)src[i] : 0.0f;
+    }
 }
 template <typename T, int R>
 __global__ void __launch_bounds__(HEAD_THREADS)
@@ -369,39 +377,16 @@ head_linear_kernel(const HoloHeadLinearArgs a, uint32_t vec) {
     float acc[R][N] = {};
     holo_pdl_wait();
     if (left) {
-        if (vec && left >= (uint32_t)N) {
-            // HEAD_BATCH weight vectors of a thread on their way at a time
-#pragma unroll 1
-            for (uint32_t k0 = kg; k0 < a.k; k0 += HEAD_BATCH * KG) {
-                uint4 raw[HEAD_BATCH];
-                float xv[HEAD_BATCH][R];
+        const bool whole = vec && left >= (uint32_t)N;
+#pragma unroll 8
+        for (uint32_t k = kg; k < a.k; k += KG) {
+            float v[N];
+            load_vec<T>(b + (uint64_t)k * a.b_ld, whole, left, v);
 #pragma unroll
-                for (int j = 0; j < HEAD_BATCH; ++j) {
-                    const uint32_t k = k0 + j * KG;
-                    raw[j] = k < a.k ? *reinterpret_cast<const uint4*>(b + (uint64_t)k * a.b_ld) : make_uint4(0, 0, 0, 0);
+            for (int r = 0; r < R; ++r) {
+                const float xv = (uint32_t)r < rows ? (float)x[(uint64_t)r * a.lda + k] : 0.0f;
 #pragma unroll
-                    for (int r = 0; r < R; ++r) xv[j][r] = k < a.k && (uint32_t)r < rows ? (float)x[(uint64_t)r * a.lda + k] : 0.0f;
-                }
-#pragma unroll
-                for (int j = 0; j < HEAD_BATCH; ++j) {
-                    if (k0 + j * KG >= a.k) break;
-                    const T* e = reinterpret_cast<const T*>(&raw[j]);
-#pragma unroll
-                    for (int r = 0; r < R; ++r)
-#pragma unroll
-                        for (int i = 0; i < N; ++i) acc[r][i] = fmaf(xv[j][r], (float)e[i], acc[r][i]);
-                }
-            }
-        } else {
-            for (uint32_t k = kg; k < a.k; k += KG) {
-                float v[N];
-                load_part<T>(b + (uint64_t)k * a.b_ld, left, v);
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const float xv = (uint32_t)r < rows ? (float)x[(uint64_t)r * a.lda + k] : 0.0f;
-#pragma unroll
-                    for (int i = 0; i < N; ++i) acc[r][i] = fmaf(xv, v[i], acc[r][i]);
-                }
+                for (int i = 0; i < N; ++i) acc[r][i] = fmaf(xv, v[i], acc[r][i]);
             }
         }
     }

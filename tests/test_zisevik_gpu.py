@@ -163,7 +163,7 @@ def test_grouped_linear(backend, dtype, tile_rows, shared, k, n, experts, tiles)
 
 
 @pytest.mark.parametrize("dtype", [F32, BF])
-@pytest.mark.parametrize("rows,heads,k,n", [(1, 3, 48, 80), (5, 2, 130, 37), (16, 4, 512, 128), (1, 16, 128, 512)])
+@pytest.mark.parametrize("rows,heads,k,n", [(1, 3, 48, 80), (5, 2, 130, 37), (16, 4, 512, 128), (1, 16, 128, 512), (1, 2, 1100, 130), (7, 2, 700, 72)])
 def test_head_linear(backend, dtype, rows, heads, k, n):
     rng = np.random.default_rng(n)
     es, lda, ld, bld = 2 if dtype == BF else 4, heads * (k + 8) + 8, heads * (n + 3), n + 8
