@@ -59,6 +59,27 @@ def test_rms_norm_multi(backend, dtype, rows, feature, step, two):
         assert not got[:, i, feature:].any()
 
 
+@pytest.mark.parametrize("dtype", [F32, BF])
+@pytest.mark.parametrize("feature,step,two", [(2048, 2048, True), (5120, 5124, True), (96, 96, False), (7, 8, True)])
+def test_rms_norm_multi_of_few_and_of_many_rows_is_the_same(backend, dtype, feature, step, two):
+    # up to one row per SM a CTA asks for its scales early; the same rows among many give the same bits
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(feature)
+    x, n = rng.standard_normal((4 * sms, feature)).astype(np.float32), 2 if two else 1
+    gammas = [rng.standard_normal(feature).astype(np.float32) for _ in range(n)]
+    got = []
+    for rows in (sms, sms + 1, 4 * sms):
+        size = rows * n * step * (2 if dtype == BF else 4)
+        ws = workspace(backend, [x[:rows]] + gammas, [size])
+        backend.dispatch(kc.KernelCall.RmsNormMulti(kc.RmsNormMultiCall(
+            kc.rb(0), kc.rb(1), kc.rb(2) if two else kc.NONE, kc.rb(1 + n), rows, feature, step, kc.f32_bits(1e-5), dtype)), ws)
+        got.append(ws.read(1 + n, size).reshape(rows, -1)[:sms])
+        ws.close()
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+
+
+
 # ---- products ----
 @pytest.mark.parametrize("dtype", [F32, BF])
 @pytest.mark.parametrize("m,w,widths,up", [
