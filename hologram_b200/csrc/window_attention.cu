@@ -330,7 +330,11 @@ latent_merge_kernel(const LatentParams p) {
     const uint32_t pair = blockIdx.x, tile = pair >> 4, row = pair / a.heads, head = pair % a.heads, tid = threadIdx.x, c = blockIdx.y * 128 + tid;
     holo_pdl_trigger();
     holo_pdl_wait();
-    // everything is requested at once: the position, and of every share that may be in use its statistics and (the first ones') values
+    const LatentRange range = latent_range(a, tile, *a.pos);
+    const uint32_t used = min(p.splits, (range.hi - range.lo + KT) / KT);
+    if (used < 2) return;
+    // one round trip for the shares' statistics and (the first ones') values. Asking for both before the position is known saves
+    // another, but most of it for nothing: at position 0 16 x 16 heads of 512 take 10.9 us, and 12.7 so
     const uint32_t ml = a.vdim + 2;
     const float* part = p.partials + (uint64_t)tile * p.splits * 16 * ml + (pair & 15u) * ml;
     float2 mine[MERGE_SPLITS / 128];
@@ -338,20 +342,14 @@ latent_merge_kernel(const LatentParams p) {
 #pragma unroll
     for (uint32_t i = 0; i < MERGE_SPLITS / 128; ++i) {
         const uint32_t share = tid + 128 * i;
-        mine[i] = share < p.splits ? *reinterpret_cast<const float2*>(part + (uint64_t)share * 16 * ml + a.vdim) : make_float2(-INFINITY, 0.0f);
+        mine[i] = share < used ? *reinterpret_cast<const float2*>(part + (uint64_t)share * 16 * ml + a.vdim) : make_float2(-INFINITY, 0.0f);
     }
 #pragma unroll
-    for (uint32_t i = 0; i < MERGE_EARLY; ++i) early[i] = c < a.vdim && i < p.splits ? part[(uint64_t)i * 16 * ml + c] : 0.0f;
-    const LatentRange range = latent_range(a, tile, *a.pos);
-    const uint32_t used = min(p.splits, (range.hi - range.lo + KT) / KT);
-    if (used < 2) return;
+    for (uint32_t i = 0; i < MERGE_EARLY; ++i) early[i] = c < a.vdim && i < used ? part[(uint64_t)i * 16 * ml + c] : 0.0f;
     const float sink = a.sink ? a.sink[head] * LOG2E : -INFINITY;
     float top = sink;
 #pragma unroll
-    for (uint32_t i = 0; i < MERGE_SPLITS / 128; ++i) {
-        if (tid + 128 * i >= used) mine[i] = make_float2(-INFINITY, 0.0f);
-        top = fmaxf(top, mine[i].x);
-    }
+    for (uint32_t i = 0; i < MERGE_SPLITS / 128; ++i) top = fmaxf(top, mine[i].x);
     for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
     if ((tid & 31u) == 0) s_red[tid >> 5] = top;
     __syncthreads();
