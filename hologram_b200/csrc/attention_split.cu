@@ -455,6 +455,12 @@ int32_t launch_sized(holo_b200_ctx* ctx, Params p, uint64_t planes, bool* taken)
     p.rowblocks = (p.rows + rb - 1) / rb;
     if (planes * p.rowblocks > 65535) return HOLO_OK;
     const uint32_t items = (uint32_t)planes * p.rowblocks;
+    // One CTA fits an SM (its ring takes 128 KB and more), so many sequences with a few keys each go round after round: 2.9 us a
+    // round for one row, 3.6 to 4.5 for several. The general routine runs several CTAs an SM: 2048 heads of 4 keys, dim 64, 25 us
+    // against 40 here; of 24 keys 45 against 41.
+    const uint64_t keys = (uint64_t)p.a.past + p.a.nnew, rounds = (items + (uint64_t)ctx->sm_count - 1) / ctx->sm_count;
+    const uint64_t ns = 400 + rounds * (p.rows == 1 ? 2900 : p.a.d <= 64 ? 3600 : 4300);
+    if (ns > holo_general_attention_ns(planes * p.rows, keys, keys, p.a.d)) return HOLO_OK;
     *taken = true;
     if (p.a.d <= 64) return rb == 1 ? launch<DT, 1, 8, 8>(ctx, p, items) : rb == 4 ? launch<DT, 4, 8, 8>(ctx, p, items) : launch<DT, 8, 8, 8>(ctx, p, items);
     if (p.a.d <= 128) return rb == 1 ? launch<DT, 1, 16, 8>(ctx, p, items) : rb == 4 ? launch<DT, 4, 16, 8>(ctx, p, items) : launch<DT, 8, 8, 16>(ctx, p, items);

@@ -238,6 +238,14 @@ struct HoloAttnArgs {
     bool all_new;     // scalar-mask form without the causal law: query row i sees every chunk row (legacy non-causal Attention)
 };
 int32_t holo_launch_decode_attention(holo_b200_ctx* ctx, const HoloAttnArgs& a);
+// What the general routine takes for a call, in ns: `rows` output rows of `keys` keys at most and `average` on average. A CTA's
+// eight warps take a key each at a time, one round trip a turn (measured 1.7 us a turn at dim 16, 1.8 at 64, 2.4 at 128, 3.5 at 256,
+// 4 us beside it); where rows fill the chip they cost 12.2 ns for one turn and 4.6 for each further one at dim 64 (14 and 6.2 at 128,
+// 17 and 9.5 at 256). The kernels that do better on long calls start and pad more: they take a call when it is worth it.
+inline uint64_t holo_general_attention_ns(uint64_t rows, uint64_t keys, uint64_t average, uint32_t d) {
+    const uint64_t vecs = (d + 31) / 32, alone = 4000 + (keys + 7) / 8 * (1300 + 280 * vecs), full = rows * (7800 + (average + 7) / 8 * (3000 + 800 * vecs)) / 1000;
+    return alone > full ? alone : full;
+}
 // attention_rows.cu: whole 16-bit sequences; *taken false: the shape is not one it serves
 int32_t holo_try_attention_tile(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool* taken);
 // attention_f32.cu: many f32 rows, with or without a cache before them

@@ -452,3 +452,52 @@ def test_chunk_of_f32_rows_after_a_cache(backend, past, valid, m, d):
     backend.dispatch(kc.KernelCall.DecodeAttentionValid(kc.DecodeAttentionValidCall(*[kc.rb(i) for i in range(7)], b, h, kv, m, past, m, d, 0, F32)), ws)
     assert norm_max_err(ws.read(6, arrs[0].nbytes, np.float32), want) <= ATTENTION_TOL[F32]
     ws.close()
+
+
+# ---- routes ----
+def times(call, tensors, monkeypatch):
+    """us of a call's launch on the device: the route that is taken, the general routine"""
+    import torch
+    be, stream, best = hb.B200Backend(0), torch.cuda.Stream(), []
+    be.set_stream(stream.cuda_stream)
+    ws = hb.DeviceWorkspace(be, len(tensors))
+    for i, t in enumerate(tensors):
+        ws.bind(i, t.data_ptr(), t.numel() * t.element_size())
+    torch.cuda.synchronize()
+    for general in (False, True):
+        if general:
+            monkeypatch.setenv("HOLO_ATTN_FORCE_GENERIC", "1")
+        low = 1e9
+        with torch.cuda.stream(stream):
+            for _ in range(5):
+                ends = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+                be.dispatch(call, ws)
+                torch.cuda._sleep(2000000)            # 1 ms: the launches are all queued before the first one starts
+                ends[0].record()
+                for _ in range(20):
+                    be.dispatch(call, ws)
+                ends[1].record()
+                stream.synchronize()
+                low = min(low, ends[0].elapsed_time(ends[1]) * 50)
+        best.append(low)
+    monkeypatch.delenv("HOLO_ATTN_FORCE_GENERIC")
+    ws.close()
+    be.close()
+    return best
+
+
+def device_tensors(shapes, dtype, seed=5):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return [torch.randn(s, generator=g, device="cuda").to({F32: torch.float32, BF: torch.bfloat16, kc.DTYPE_F16: torch.float16}[dtype]) for s in shapes]
+
+
+@pytest.mark.parametrize("b,h,kv,past,d,dtype", [(64, 32, 32, 3, 64, F32), (64, 32, 32, 7, 64, BF), (256, 12, 12, 3, 128, BF), (32, 12, 12, 3, 64, kc.DTYPE_F16),
+                                                 (64, 32, 32, 23, 64, F32), (16, 32, 8, 3, 64, F32), (1, 12, 2, 3, 128, F32)])
+def test_one_row_of_many_short_caches_takes_the_quicker_route(monkeypatch, b, h, kv, past, d, dtype):
+    # the split kernel took 40 us on the first call, the general routine 25: it must not lose more than the 15 % that boxes and estimates differ by
+    import torch
+    x = device_tensors([(b, h, 1, d), (b, kv, past, d), (b, kv, past, d), (b, kv, 1, d), (b, kv, 1, d)], dtype)
+    x += [torch.tensor([past], dtype=torch.int32, device="cuda"), torch.empty_like(x[0])]
+    now, general = times(kc.KernelCall.DecodeAttentionValid(kc.DecodeAttentionValidCall(*[kc.rb(i) for i in range(7)], b, h, kv, 1, past, 1, d, 0, dtype)), x, monkeypatch)
+    assert now <= 1.15 * general, (now, general)
