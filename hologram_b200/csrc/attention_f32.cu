@@ -274,9 +274,19 @@ int32_t holo_try_attention_f32(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool* 
     if (((cache | (uintptr_t)a.q | (uintptr_t)a.k_new | (uintptr_t)a.v_new | (uintptr_t)a.out) & 15u) != 0) return HOLO_OK;
     const uint64_t planes = (uint64_t)a.b * a.h, blocks = ((uint64_t)a.m + 63) / 64;
     if (planes * a.m > 0x7fffffffull || 2 * blocks > 65535 || (uint64_t)a.past + a.nnew > 0x7fffffffull) return HOLO_OK;
+    // where 64-row blocks leave SMs without one: 32-row blocks whose four groups share the keys
+    const uint64_t sms = (uint64_t)ctx->sm_count, keys = (uint64_t)a.past + a.nnew, tiles = (keys + TILE - 1) / TILE;
+    const bool small = a.d <= 64 && planes * blocks < sms;
+    // Rows and keys are padded to whole tiles, so a few rows of a few keys are the general routine's. Measured, in ns: a wave of CTAs
+    // and its first pass over a group's tile, then each further pass; dims up to 64 with every SM full, 31 a CTA and tile.
+    auto waves = [&](uint64_t rows) { return (planes * ((a.m + rows - 1) / rows) + sms - 1) / sms; };
+    const uint64_t ns = small ? waves(32) * (8300 + ((tiles + 3) / 4 - 1) * 9500) : a.d <= 64 ? 6000 + planes * blocks * tiles * 31 * 148 / sms
+                              : a.d <= 96 ? waves(64) * (10300 + ((tiles + 1) / 2 - 1) * 12500) : waves(64) * (12500 + ((tiles + 1) / 2 - 1) * 15800);
+    const uint64_t average = (uint64_t)a.past + (a.all_new ? a.m : (a.m + 1) / 2);
+    // within 8 % the estimates do not tell which: this kernel
+    if (ns * 25 > holo_general_attention_ns(planes * a.m, keys, average, a.d) * 27) return HOLO_OK;
     *taken = true;
     const uint32_t n = (uint32_t)planes;
-    // where 64-row blocks leave SMs without one: 32-row blocks whose four groups share the keys
-    if (a.d <= 64) return planes * blocks < (uint64_t)ctx->sm_count ? launch<64, 2, 4>(ctx, a, n) : launch<64, 4, 1>(ctx, a, n);
+    if (a.d <= 64) return small ? launch<64, 2, 4>(ctx, a, n) : launch<64, 4, 1>(ctx, a, n);
     return a.d <= 96 ? launch<96, 4, 2>(ctx, a, n) : launch<128, 4, 2>(ctx, a, n);
 }

@@ -501,3 +501,14 @@ def test_one_row_of_many_short_caches_takes_the_quicker_route(monkeypatch, b, h,
     x += [torch.tensor([past], dtype=torch.int32, device="cuda"), torch.empty_like(x[0])]
     now, general = times(kc.KernelCall.DecodeAttentionValid(kc.DecodeAttentionValidCall(*[kc.rb(i) for i in range(7)], b, h, kv, 1, past, 1, d, 0, dtype)), x, monkeypatch)
     assert now <= 1.15 * general, (now, general)
+
+
+@pytest.mark.parametrize("b,h,kv,s,d,causal", [(64, 32, 32, 2, 128, True), (32, 32, 32, 2, 64, False), (1, 12, 12, 8, 128, True), (1, 12, 12, 4, 64, False),
+                                               (1, 12, 12, 8, 96, True), (32, 32, 32, 4, 128, False), (1, 12, 12, 64, 64, True), (32, 32, 32, 16, 96, True)])
+def test_a_few_f32_rows_take_the_quicker_route(monkeypatch, b, h, kv, s, d, causal):
+    # tiles of 64 keys and of 32 or 64 rows took 167 us on the first call, the general routine 52
+    import torch
+    x = device_tensors([(b, h, s, d), (b, kv, s, d), (b, kv, s, d)], F32)
+    x.append(torch.empty_like(x[0]))
+    now, general = times(kc.KernelCall.Attention(kc.AttentionCall(*[kc.rb(i) for i in range(4)], b, h, s, d, 0, int(causal), 0, F32)), x, monkeypatch)
+    assert now <= 1.15 * general, (now, general)
