@@ -297,6 +297,42 @@ __global__ void __launch_bounds__(THREADS) matmul_cell_kernel(const Params p) {
     }
 }
 
+// One thread per cell, operands from global memory: nothing to fill or to wait for
+constexpr uint32_t THREAD_COLS = 128;
+template <int DT>
+__global__ void __launch_bounds__(THREAD_COLS) matmul_thread_kernel(const Params p) {
+    holo_pdl_trigger();
+    holo_pdl_wait();
+    const uint32_t j = blockIdx.x * THREAD_COLS + threadIdx.x, i = blockIdx.y;
+    if (j >= p.n) return;
+    const bool fused = j < p.n8;
+    float acc = 0.0f;
+    for (uint32_t kk = 0; kk < p.k; ++kk) {
+        const float a = holo::load_float(p.a, (uint64_t)i * p.k + kk, DT), b = holo::load_float(p.b, (uint64_t)kk * p.n + j, DT);
+        acc = fused ? __fmaf_rn(a, b, acc) : __fadd_rn(acc, __fmul_rn(a, b));
+    }
+    store_cell<DT>(p, acc, (uint64_t)i * p.n + j);
+}
+
+// Where that is the quicker one. Short chains do not pay for the ring: us, a thread per cell / tiles, f32 1 x 4 x 1001 1.4 / 1.8,
+// 300 x 4 x 129 1.8 / 2.4, f16 300 x 1 x 2001 5.8 / 15; the lines are where enough cells or depth share a tile. With up to 8 rows the
+// product is a pass over B, and the wider B is the deeper it may be before a 4 x 32 tile, three quarters of it idle for one row, is
+// the better way to read it: f32 1 x 201 x 100001 15 / 32, 8 x 33 x 100001 10.6 / 16.4, 8 x 404 x 100001 131 / 121.
+template <int DT>
+bool thread_per_cell(const Params& p) {
+    constexpr bool F16 = DT == HOLO_DTYPE_F16;      // widening f16 takes a dozen instructions, which a tile does once
+    const uint64_t cells = (uint64_t)p.m * p.n;
+    if (p.m <= 8) {
+        if (F16) return p.k <= 10 + (p.m == 1 ? p.n / 2500 : min(p.n / 3500, 28u));
+        if (p.m == 1 && p.n >= 100000) return true;
+        return p.k <= 16 + (p.m <= 2 ? p.n / (700 * p.m) : min(p.n / 1500, 104u));
+    }
+    if (p.n < 8) return p.k <= 4 && p.m <= 1000;
+    if (F16) return p.m <= 4000 && cells <= 800000 && p.k <= (cells >= 40000 ? 12u : 6u);
+    if (DT == HOLO_DTYPE_BF16) return p.m <= 1200 && cells <= 800000 && p.k <= 20;
+    return p.m <= 2001 && cells <= (p.m <= 64 ? 400000u : 200000u) && p.k <= 24;
+}
+
 template <int DT, int BM, int BN, int BK, int TM, int TN, int KU, int THREADS>
 int32_t launch(holo_b200_ctx* ctx, Params p) {
     constexpr int STAGES = DT == HOLO_DTYPE_F32 ? 3 : 2;
@@ -316,13 +352,18 @@ int32_t launch(holo_b200_ctx* ctx, Params p) {
     return HOLO_OK;
 }
 
-// Which tile: few rows are bound by the chain's latency and by the weight's way to shared memory (4 rows, deep steps); up to
+// Which kernel: see above; else which tile: few rows are bound by the chain's latency and by the weight's way to shared memory (4 rows, deep steps); up to
 // one 16 x 32 tile per SM four warps share each; more of them fill an SM several deep with two warps each; large products
 // spend fewest reads of shared memory in 64 x 32 tiles. Measured f32, us, in this order (the one taken in brackets):
 // 1 x 1024 x 1024 [7.7] 12.1 14.0 25.3; 32 x 1000 x 771 21.9 [15.0] 17.5 26.3; 512^3 29.0 16.2 [16.0] 32.7;
 // 500 x 1000 x 771 106 46.5 [35.9] 65.7; 381 x 768 x 3072 179 67.7 55.4 [50.6]; 1000 x 2048 x 2048 825 299 237 [209].
 template <int DT>
 int32_t launch_sized(holo_b200_ctx* ctx, const Params& p) {
+    if (thread_per_cell<DT>(p)) {
+        HOLO_CUDA(holo_launch_kernel(ctx, matmul_thread_kernel<DT>, dim3((p.n + THREAD_COLS - 1) / THREAD_COLS, p.m), dim3(THREAD_COLS), 0, 1, p));
+        ctx->launches++;
+        return HOLO_OK;
+    }
     const uint64_t sms = (uint64_t)ctx->sm_count;
     auto tiles = [&](uint64_t bm, uint64_t bn) { return (p.m + bm - 1) / bm * ((p.n + bn - 1) / bn); };
     if (p.m <= 8) return launch<DT, 4, 32, 128, 1, 1, 16, 128>(ctx, p);

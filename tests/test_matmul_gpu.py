@@ -181,12 +181,15 @@ def test_f32_matmul_is_the_reference_recurrence(backend, m, k, n):
 
 @pytest.mark.parametrize("dtype", [kc.DTYPE_F32, BF, kc.DTYPE_F16])
 @pytest.mark.parametrize("m,k,n", [(1, 1, 1), (1, 33, 41), (3, 31, 1003), (5, 100, 64), (16, 37, 531), (33, 65, 130), (129, 7, 8 * 37), (200, 70, 2055),
-                                   (500, 50, 771), (1025, 36, 1801), (4, 96, 7)])
+                                   (500, 50, 771), (1025, 36, 1801), (4, 96, 7),
+                                   # every ring goes round: four full steps of k and a part of one, 16-byte copies and single ones
+                                   (5, 645, 1003), (8, 772, 516), (33, 389, 130), (40, 324, 268), (300, 323, 771), (300, 388, 772), (1025, 197, 1801), (1100, 196, 1804),
+                                   # one thread per cell and its neighbours: short chains, few rows of a wide B
+                                   (1, 9, 100001), (1, 150, 100001), (3, 60, 100001), (8, 81, 60000), (2, 100, 60000), (9, 12, 2001), (9, 20, 33), (64, 24, 517), (64, 25, 517),
+                                   (300, 4, 7), (300, 12, 1001), (1200, 20, 65), (2001, 12, 33)])
 def test_every_tile_of_the_per_cell_kernel_is_bit_exact(backend, dtype, m, k, n):
     # edges of the tiles and of the k steps, pitches that are multiples of four elements and that are not, columns of the
     # multiply-then-add tail alone and beside full tiles, chains whose sums are -0 and subnormal
-    if dtype != kc.DTYPE_F32 and k % 8 == 0 and n % 8 == 0:
-        pytest.skip("tensor-core shape")
     rng = np.random.default_rng(m + 3 * k + 5 * n)
     a, b, r = rng.standard_normal(m * k, dtype=np.float32), rng.standard_normal(k * n, dtype=np.float32), rng.standard_normal(m * n, dtype=np.float32)
     if dtype == kc.DTYPE_F32:
