@@ -44,7 +44,7 @@ __device__ __forceinline__ float f16_to_f32(uint16_t h) {
 __device__ __forceinline__ uint16_t f32_to_f16_ref(float v) {
     const uint32_t bits = __float_as_uint(v), size = bits & 0x7fffffffu;
     const uint32_t normal = (size - 0x38000000u + 0x1000u) >> 13;
-    const uint32_t shift = min(126u - (size >> 23), 31u), small = (((size & 0x7fffffu) | 0x800000u) + (1u << (shift - 1))) >> shift;
+    const uint32_t half = min(125u - (size >> 23), 30u), small = (((size & 0x7fffffu) | 0x800000u) + (1u << half)) >> (half + 1);
     const uint32_t large = size > 0x7f800000u ? 0x7e00u : 0x7c00u;
     return (uint16_t)((bits >> 16 & 0x8000u) | (size < 0x38800000u ? small : size < 0x47800000u ? normal : large));
 }
