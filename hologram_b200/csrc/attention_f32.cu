@@ -8,9 +8,7 @@
 // Measured, us (one CTA per query row, before, in brackets): 381 rows, 12 heads, dim 64 20 [994]; 512 rows 44 [1720]; 1024 rows, 32
 // heads over 8, dim 128, causal 272 [11461]; two such sequences, all keys 949 [47527] = 36 TFLOP/s of 74.
 //
-// A zero weight times an infinite or NaN value is NaN, so a masked key could reach rows that must not see it. All such cases end
-// in an output that is not finite: the CTA then redoes its rows with the general row routine, which defines the result.
-#include "attention_generic.cuh"
+// A weight of zero times an infinite or NaN value is NaN: keys that only some rows of a warp see are added row by row.
 #include "common.h"
 #include "numerics.cuh"
 
@@ -51,15 +49,14 @@ struct Layout {
     static constexpr int ROWS = 16 * NR, WARPS = NR * NG, LD = D + 4;
     static constexpr int Q = ROWS * LD, GROUP = TILE * LD + TILE * D, P = WARPS * 16 * P_LD;
     static constexpr int FLOATS = Q + NG * GROUP + P;
-    static_assert(NG * ROWS * (D + 2) <= NG * GROUP && WARPS * (D + 2) <= NG * GROUP, "the groups' results and the row routine fit in the tiles' memory");
+    static_assert(NG * ROWS * (D + 2) <= NG * GROUP, "the groups' results fit in the tiles' memory");
 };
 
-template <int D, int NR, int NG>
+template <int D, int NR, int NG, bool CAUSAL>
 __global__ void __launch_bounds__(NR * NG * 32, NR * NG <= 4 ? 3 : 1)
 attention_f32_kernel(const __grid_constant__ HoloAttnArgs a) {
     using L = Layout<D, NR, NG>;
     extern __shared__ __align__(16) float smem[];
-    __shared__ uint32_t s_redo;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, group = warp / NR, wrow = warp % NR;
     // lanes' bits in the order column, row, column, column, row: 128-bit reads then take two wavefronts
     const uint32_t tx = (lane & 1) | ((lane >> 1) & 6), ty = ((lane >> 1) & 1) | ((lane >> 3) & 2);
@@ -72,7 +69,6 @@ attention_f32_kernel(const __grid_constant__ HoloAttnArgs a) {
     const uint32_t past = a.valid_len ? min(*a.valid_len, a.past) : a.past;
     auto limit_of = [&](uint32_t row) { return past + (a.all_new ? a.nnew : min(row + 1, a.nnew)); };
     const uint32_t keys = limit_of(min(row0 + L::ROWS, a.m) - 1), tiles = (keys + TILE - 1) / TILE, dvec = a.d / 4;
-    if (tid == 0) s_redo = 0;
     {
         const float* q = (const float*)a.q + ((uint64_t)plane * a.m + row0) * a.d;
         for (uint32_t i = tid; i < L::ROWS * (D / 4); i += L::WARPS * 32) {
@@ -181,8 +177,17 @@ attention_f32_kernel(const __grid_constant__ HoloAttnArgs a) {
         meet();         // V is here, and everybody in the group has left K
         if (t + NG < tiles) request(s_k, L::LD, a.k_past, a.k_new, t + NG);
         commit();
+        // Keys of this tile that all rows of the warp see (those of its first row, in lane 0) and that any of them does (its last row: ty
+        // 3, lane 18); without the causal law all of them, rows of zeros behind the last one included.
+        const uint32_t at = t * TILE;
+        uint32_t common = TILE, end = TILE;
+        if constexpr (CAUSAL) {
+            const uint32_t all_see = __shfl_sync(0xffffffffu, limit[0], 0), one_sees = __shfl_sync(0xffffffffu, limit[3], 18);
+            end = one_sees > at ? min(one_sees - at, (uint32_t)TILE) : 0u;
+            common = all_see > at ? min(all_see - at, (uint32_t)TILE) & ~3u : 0u;
+        }
 #pragma unroll 1
-        for (int j = 0; j < TILE; j += 4) {
+        for (uint32_t j = 0; j < common; j += 4) {
             float4 w[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(s_p + (ty + 4 * i) * P_LD + j);
@@ -200,6 +205,29 @@ attention_f32_kernel(const __grid_constant__ HoloAttnArgs a) {
                         o[i][2 * c + 1] = fma2(w2, v[c].y, o[i][2 * c + 1]);
                     }
                 }
+            }
+        }
+        if constexpr (CAUSAL)
+#pragma unroll 1
+        for (uint32_t j = common; j < end; j += 4) {
+            float4 w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(s_p + (ty + 4 * i) * P_LD + j);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                ulonglong2 v[D / 32];
+#pragma unroll
+                for (int c = 0; c < D / 32; ++c) v[c] = *reinterpret_cast<const ulonglong2*>(s_v + (j + e) * D + 32 * c + 4 * tx);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (at + j + e < limit[i]) {
+                        const uint64_t w2 = both(e == 0 ? w[i].x : e == 1 ? w[i].y : e == 2 ? w[i].z : w[i].w);
+#pragma unroll
+                        for (int c = 0; c < D / 32; ++c) {
+                            o[i][2 * c] = fma2(w2, v[c].x, o[i][2 * c]);
+                            o[i][2 * c + 1] = fma2(w2, v[c].y, o[i][2 * c + 1]);
+                        }
+                    }
             }
         }
         __syncwarp();   // the warp's weights have been read
@@ -224,7 +252,6 @@ attention_f32_kernel(const __grid_constant__ HoloAttnArgs a) {
     __syncthreads();
     float* out = (float*)a.out + ((uint64_t)plane * a.m + row0) * a.d;
     const uint32_t here = min((uint32_t)L::ROWS, a.m - row0);
-    bool finite = true;
     for (uint32_t i = tid; i < here * dvec; i += L::WARPS * 32) {
         const uint32_t r = i / dvec, c = 4 * (i % dvec);
         float most = -INFINITY, total = 0.0f;
@@ -238,31 +265,26 @@ attention_f32_kernel(const __grid_constant__ HoloAttnArgs a) {
             total = fmaf(f, s_ml[2 * (g * L::ROWS + r) + 1], total);
             acc = make_float4(fmaf(f, v.x, acc.x), fmaf(f, v.y, acc.y), fmaf(f, v.z, acc.z), fmaf(f, v.w, acc.w));
         }
-        const float4 v = make_float4(acc.x / total, acc.y / total, acc.z / total, acc.w / total);
-        finite = finite && isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w);
-        *reinterpret_cast<float4*>(out + (uint64_t)r * a.d + c) = v;
+        *reinterpret_cast<float4*>(out + (uint64_t)r * a.d + c) = make_float4(acc.x / total, acc.y / total, acc.z / total, acc.w / total);
     }
-    if (!finite) s_redo = 1;
-    __syncthreads();
-    if (s_redo)
-        for (uint32_t r = 0; r < here; ++r) {
-            holo_attn::attention_row<false, L::WARPS>(a, plane * a.m + row0 + r, s_o);
-            __syncthreads();
-        }
 }
 
-template <int D, int NR, int NG>
-int32_t launch(holo_b200_ctx* ctx, const HoloAttnArgs& a, uint32_t planes) {
+template <int D, int NR, int NG, bool CAUSAL>
+int32_t launch_form(holo_b200_ctx* ctx, const HoloAttnArgs& a, uint32_t planes) {
     using L = Layout<D, NR, NG>;
     constexpr int SMEM = L::FLOATS * 4;
     static thread_local int configured_device = -1;
     if (configured_device != ctx->device) {
-        HOLO_CUDA(cudaFuncSetAttribute(attention_f32_kernel<D, NR, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        HOLO_CUDA(cudaFuncSetAttribute(attention_f32_kernel<D, NR, NG, CAUSAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
         configured_device = ctx->device;
     }
-    HOLO_CUDA(holo_launch_kernel(ctx, attention_f32_kernel<D, NR, NG>, dim3(planes, (a.m + L::ROWS - 1) / L::ROWS), dim3(L::WARPS * 32), SMEM, 1, a));
+    HOLO_CUDA(holo_launch_kernel(ctx, attention_f32_kernel<D, NR, NG, CAUSAL>, dim3(planes, (a.m + L::ROWS - 1) / L::ROWS), dim3(L::WARPS * 32), SMEM, 1, a));
     ctx->launches++;
     return HOLO_OK;
+}
+template <int D, int NR, int NG>
+int32_t launch(holo_b200_ctx* ctx, const HoloAttnArgs& a, uint32_t planes) {
+    return a.all_new ? launch_form<D, NR, NG, false>(ctx, a, planes) : launch_form<D, NR, NG, true>(ctx, a, planes);
 }
 
 }  // namespace

@@ -454,6 +454,40 @@ def test_chunk_of_f32_rows_after_a_cache(backend, past, valid, m, d):
     ws.close()
 
 
+SPECIAL = {BF: (0x7f80, 0xff80, 0x7fc0), kc.DTYPE_F16: (0x7c00, 0xfc00, 0x7e00), F32: (np.inf, -np.inf, np.nan)}
+
+
+def same_as_general(backend, monkeypatch, run, dtype):
+    """A route's output and the general routine's: NaN and infinities in the same places, other values within the tolerance."""
+    got = wide(run(), dtype)
+    monkeypatch.setenv("HOLO_ATTN_FORCE_GENERIC", "1")
+    want = wide(run(), dtype)
+    monkeypatch.delenv("HOLO_ATTN_FORCE_GENERIC")
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    fine = np.isfinite(want)
+    assert fine.any() and not fine.all() and np.isinf(want).any() and np.isnan(want).any()
+    assert np.max(np.abs(got[fine] - want[fine])) <= ATTENTION_TOL[dtype] * np.max(np.abs(want[fine]))
+
+
+@pytest.mark.parametrize("dtype", [F32])
+@pytest.mark.parametrize("b,h,kv,s,d,causal,sigma", [(1, 4, 2, 200, 64, True, 1.0), (1, 4, 2, 131, 64, False, 6.0), (2, 3, 3, 70, 128, True, 6.0), (1, 2, 2, 300, 128, False, 1.0),
+                                                     (1, 80, 4, 300, 48, True, 1.0), (1, 4, 4, 260, 80, True, 1.0)])
+def test_infinities_and_nan_reach_the_rows_that_see_them(backend, monkeypatch, dtype, b, h, kv, s, d, causal, sigma):
+    # infinite values of both signs in one column, in a column each, a value row of NaN, a NaN key, a query and a key whose product is infinite
+    q, k, v = attention_inputs(b, h, kv, s, d, dtype, 3 * s + d, sigma)
+    inf, ninf, nan = SPECIAL[dtype]
+    q4, k4, v4 = q.reshape(b, h, s, d), k.reshape(b, kv, s, d), v.reshape(b, kv, s, d)
+    v4[0, 0, 5, 2], v4[0, 0, s // 2, 2], v4[0, 0, s // 3, 7], v4[0, 0, s - 2, 9] = inf, ninf, ninf, inf
+    if causal:
+        v4[0, kv - 1, s - 20] = nan
+        k4[0, kv - 1, s - 9, 1] = nan
+    big = {F32: 3e38, BF: 0x7f61, kc.DTYPE_F16: inf}[dtype]     # 3e38; its square, and an infinity times anything but zero, is infinite
+    q4[b - 1, h - 1, s - 30, 0] = big
+    k4[b - 1, kv - 1, 17, 0] = big
+    same_as_general(backend, monkeypatch, lambda: run_attention(backend, q, k, v, b, h, kv, s, d, causal, dtype), dtype)
+
+
+
 # ---- routes ----
 def times(call, tensors, monkeypatch):
     """us of a call's launch on the device: the route that is taken, the general routine"""
@@ -511,4 +545,16 @@ def test_a_few_f32_rows_take_the_quicker_route(monkeypatch, b, h, kv, s, d, caus
     x = device_tensors([(b, h, s, d), (b, kv, s, d), (b, kv, s, d)], F32)
     x.append(torch.empty_like(x[0]))
     now, general = times(kc.KernelCall.Attention(kc.AttentionCall(*[kc.rb(i) for i in range(4)], b, h, s, d, 0, int(causal), 0, F32)), x, monkeypatch)
+    assert now <= 1.15 * general, (now, general)
+
+
+@pytest.mark.parametrize("dtype", [F32])
+@pytest.mark.parametrize("b,h,kv,s,d,causal", [(1, 12, 12, 128, 64, True), (1, 1, 1, 128, 128, False), (1, 8, 8, 381, 64, True), (1, 32, 8, 512, 128, False)])
+def test_a_value_that_is_not_finite_costs_no_more_than_the_general_routine(monkeypatch, b, h, kv, s, d, causal, dtype):
+    # every row sees it, in one column: f32, 12 heads of 128 rows took 718 us where the general routine takes 87
+    import torch
+    x = device_tensors([(b, h, s, d), (b, kv, s, d), (b, kv, s, d)], dtype)
+    x[2][:, :, 0, 3] = float("inf")
+    x.append(torch.empty_like(x[0]))
+    now, general = times(kc.KernelCall.Attention(kc.AttentionCall(*[kc.rb(i) for i in range(4)], b, h, s, d, kv if kv != h else 0, int(causal), 0, dtype)), x, monkeypatch)
     assert now <= 1.15 * general, (now, general)
