@@ -24,9 +24,13 @@ __device__ __forceinline__ float kv_elem(const void* base, const float* scales, 
     }
 }
 
-// Output row r = (batch, head, query row), by all WARPS warps of the block; s_mem holds [WARPS][d + 2].
-template <bool Q8, int WARPS>
-__device__ __forceinline__ void attention_row(const HoloAttnArgs& a, const uint32_t r, float* s_mem) {
+template <bool Q8>
+__global__ void __launch_bounds__(GEN_WARPS * 32)
+decode_attention_generic_kernel(HoloAttnArgs a) {
+    holo_pdl_trigger();
+    holo_pdl_wait();
+    extern __shared__ float s_mem[];  // [GEN_WARPS][d + 2]
+    const uint32_t r = blockIdx.x;    // output row: (batch, head, query row)
     const uint32_t d = a.d, h = a.h, m = a.m, hkv = a.hkv;
     const uint32_t bi = r / (h * m), hi = (r / m) % h, qi = r % m;
     const uint32_t kvh = bi * hkv + hi / (h / hkv);
@@ -47,7 +51,7 @@ __device__ __forceinline__ void attention_row(const HoloAttnArgs& a, const uint3
         o[i] = 0.0f;
     }
     float mx = -INFINITY, sum = 0.0f;
-    for (uint32_t kj = warp; kj < vis; kj += WARPS) {
+    for (uint32_t kj = warp; kj < vis; kj += GEN_WARPS) {
         const bool past = kj < vis_past;
         const void* kb = past ? a.k_past : a.k_new;
         const void* vb = past ? a.v_past : a.v_new;
@@ -89,16 +93,16 @@ __device__ __forceinline__ void attention_row(const HoloAttnArgs& a, const uint3
     }
     __syncthreads();
     float gm = -INFINITY;
-    for (int w = 0; w < WARPS; ++w) gm = fmaxf(gm, s_mem[(size_t)w * (d + 2) + d]);
+    for (int w = 0; w < GEN_WARPS; ++w) gm = fmaxf(gm, s_mem[(size_t)w * (d + 2) + d]);
     float gs = 0.0f;
-    for (int w = 0; w < WARPS; ++w) {
+    for (int w = 0; w < GEN_WARPS; ++w) {
         float wm = s_mem[(size_t)w * (d + 2) + d];
         if (wm != -INFINITY) gs += s_mem[(size_t)w * (d + 2) + d + 1] * expf(wm - gm);
     }
     const float denom = fmaxf(gs, 1e-30f);
     for (uint32_t c = threadIdx.x; c < d; c += blockDim.x) {
         float acc = 0.0f;
-        for (int w = 0; w < WARPS; ++w) {
+        for (int w = 0; w < GEN_WARPS; ++w) {
             float wm = s_mem[(size_t)w * (d + 2) + d];
             if (wm != -INFINITY) acc += s_mem[(size_t)w * (d + 2) + c] * expf(wm - gm);
         }
@@ -106,15 +110,6 @@ __device__ __forceinline__ void attention_row(const HoloAttnArgs& a, const uint3
         // (cpu/float_kernels.rs:3851-3854, 2451-2454)
         holo::store_float(a.out, (uint64_t)r * d + c, (vis == 0 || gm == -INFINITY) ? 0.0f : acc / denom, a.dtype);
     }
-}
-
-template <bool Q8>
-__global__ void __launch_bounds__(GEN_WARPS * 32)
-decode_attention_generic_kernel(HoloAttnArgs a) {
-    holo_pdl_trigger();
-    holo_pdl_wait();
-    extern __shared__ float s_mem[];
-    attention_row<Q8, GEN_WARPS>(a, blockIdx.x, s_mem);
 }
 
 }  // namespace holo_attn

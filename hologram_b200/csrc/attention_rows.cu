@@ -5,18 +5,20 @@
 //   warp 1     tcgen05.mma issuer: S = Q K^T, then O += P V with P read from TMEM, the two query tiles in turn
 //   warps 2-9  softmax, one group of four warps per query tile, one thread per row: running maximum, exponentials, row sum;
 //              a row's O is rescaled in TMEM only when its maximum grows by more than 2^GROWTH
-// The weights are f32 values, and 16 bits of them would not do: each goes to the tensor core as two 16-bit terms (the rounded
-// value and the rounded remainder: 2^-18 relative in bf16, 2^-22 in f16, below what a chain of f32 additions over the keys loses),
-// so O costs two products. Scores need no split: products of 16-bit values are exact in f32.
+// The weights are f32 values, and 16 bits of them would not do: each goes to the tensor core as two 16-bit terms, the rounded value
+// and the rounded remainder, so O costs two products. That holds a weight to 2^-17 of itself in bf16 and to 2^-23 in f16 (f32: 2^-24),
+// and the tensor core's sums over long sequences lose about 2^-18 more. It is less than the general routine keeps, whose weights and
+// sums are f32; what shows is the output's own 16 bits. Error against 64 bits, here / there, normal inputs: bf16 16 keys 0.003279 /
+// 0.003283, 512 causal 0.003178 / 0.003177, 2048 0.003321 / 0.003317; f16 0.0002061 / 0.0002061, 0.0001992 / 0.0001992, 0.0002077 /
+// 0.0002076. Scores need no split: products of 16-bit values are exact in f32.
 // TMEM (512 columns): S at 0 and 128, overwritten by its weights (first terms, then second terms), O at 256 and 384.
 // Bound: three products per score on the tensor core (1536 cycles a 128 x 128 tile at dim 128) against 1024 cycles of ex2.
 // 2048 rows, 32 heads over 8, dim 128, causal, bf16: one CTA per row on the CUDA cores took 48450 us, this 68 us (the tensor
 // core's share 24 us). Error against 64 bits 0.0032 in both: the output's own 16 bits.
 //
-// A zero weight times an infinite or NaN value is NaN, so a masked key could reach rows that must not see it. All such cases
-// end in an output that is not finite: the CTA then redoes its rows with the general row routine, which defines the result.
+// A weight of zero times an infinite or NaN value is NaN, and so is the sum of an infinite value's two terms: a value that is not
+// finite spoils its column of O in every row of the tile. compute_again sets that right.
 #include "attention_tile.cuh"
-#include "attention_generic.cuh"
 
 namespace {
 
@@ -56,6 +58,164 @@ __device__ __forceinline__ void split_weights(float x, float y, uint32_t& first,
 }
 
 template <bool F16>
+__device__ __forceinline__ float2 widen_pair(uint32_t v) {
+    return F16 ? widen_f16(v) : make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
+
+// Shared memory behind the tiles: barriers from `bars` on, flags, then what a row's weights refer to and what is to be computed again of it
+struct RowsTail {
+    uint32_t q, k, v, bars;     // offsets
+    __device__ __forceinline__ RowsTail(uint32_t nq, uint32_t tile_bytes) : q(0), k(nq * tile_bytes), v(k + 2 * tile_bytes), bars(v + 2 * tile_bytes) {}
+    static constexpr uint32_t AGAIN_BAR = 120, AGAIN_SCORES_BAR = 128, TMEM = 144, ABORT = 148, AGAIN = 152, SPOILT = 160, ROWS = 256, BYTES = 256 + 256 * 8;
+};
+enum { ROW_STAYS = 0, ROW_COLUMNS = 1, ROW_ALL = 2 };
+constexpr float WILD = 0x1p22f;     // from here on rounding moves exponents of two by whole units: weights no longer have the range that the tiles count on
+
+// Columns that are not finite in a row whose sum is, and whole rows with a sum that is not or with exponents beyond WILD: scores by
+// another product, weights in f32, only the keys that a row sees, one thread a row. All threads come here, with every load and product
+// at its end; nobody leaves early, they meet after each tile. One column of 2048 rows, 32 heads over 8, dim 128, causal: 285 us instead
+// of 69 (redoing the rows one after another 124000, the general routine 48400); 12 heads x 128 rows, dim 64 19 instead of 6.7 (1580,
+// 90); 16 rows 12 instead of 5.7 (89, 9).
+template <bool F16>
+__device__ __noinline__ void compute_again(const CUtensorMap& map_k, const CUtensorMap& map_v, const RowsParams& p, uint8_t* sm, uint32_t tmem_base, uint32_t row0,
+                                           uint32_t n0, uint32_t n1) {
+    const HoloAttnArgs& a = p.a;
+    const uint32_t tile_bytes = p.chunks * TILE_CHUNK, base = smem_u32(sm), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const RowsTail at(p.nq, tile_bytes);
+    const uint32_t bar = base + at.bars + RowsTail::AGAIN_BAR, bar_s = base + at.bars + RowsTail::AGAIN_SCORES_BAR;
+    volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(sm + at.bars + RowsTail::ABORT);
+    uint32_t* s_spoilt = reinterpret_cast<uint32_t*>(sm + at.bars + RowsTail::SPOILT);      // a bit per column
+    const uint32_t plane = blockIdx.x, kv_plane = plane / a.h * a.hkv + plane % a.h / (a.h / a.hkv);
+    const uint32_t q = warp < 2 ? 0u : (warp - 2) >> 2, quarter = warp & 3u, row = row0 + q * 128 + quarter * 32 + lane, n = warp < 2 ? 0u : q ? n1 : n0;
+    const uint32_t limit = a.all_new ? a.m : min(row + 1, a.m), seen = a.all_new ? a.m : min(row - lane + 32, a.m);     // keys of this row, of any row of the warp
+    const uint32_t tmem_s = tmem_base + q * 128 + ((quarter * 32u) << 16), tmem_o = tmem_s + 256;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    float top = 0.0f, sum = 0.0f;
+    uint32_t mine[4] = {0, 0, 0, 0};
+    if (n) {
+        const float2 about = reinterpret_cast<const float2*>(sm + at.bars + RowsTail::ROWS)[threadIdx.x - 64];
+        top = about.x;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            if (16 * g >= a.d) break;
+            uint32_t o[16], bits = 0;
+            tmem_ld16(tmem_o + 16 * g, o);
+#pragma unroll
+            for (int x = 0; x < 16; ++x)
+                if (about.y == ROW_ALL || !isfinite(__uint_as_float(o[x]))) bits |= 1u << x;
+            if (about.y != ROW_STAYS) mine[g >> 1] |= bits << (16 * (g & 1));
+        }
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+            if (mine[w]) atomicOr(s_spoilt + w, mine[w]);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    auto spoilt = [&](uint32_t g) { return (s_spoilt[g >> 1] >> (16 * (g & 1u)) & 0xffffu) != 0; };
+#pragma unroll 1
+    for (uint32_t t = 0; t < max(n0, n1); ++t) {
+        if (threadIdx.x == 0 && !*s_abort) {
+            mbar_arrive_expect_tx(bar, 2 * tile_bytes);
+            for (uint32_t c = 0; c < p.chunks; ++c) {
+                tma_load_3d(base + at.k + c * TILE_CHUNK, &map_k, (int)(64 * c), (int)(t * 128), (int)kv_plane, bar);
+                tma_load_3d(base + at.v + c * TILE_CHUNK, &map_v, (int)(64 * c), (int)(t * 128), (int)kv_plane, bar);
+            }
+            if (mbar_wait(bar, t & 1u, s_abort, p.status)) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t idesc = (1u << 4) | (F16 ? 0u : (1u << 7) | (1u << 10)) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+                const uint64_t dq = smem_desc(base + at.q, 16, 1024), dk = smem_desc(base + at.k, 16, 1024);
+                for (uint32_t i = 0; i < 2; ++i)
+                    for (uint32_t k = 0; t < (i ? n1 : n0) && k < a.d / 16; ++k) {
+                        const uint32_t off = (k >> 2) * (TILE_CHUNK >> 4) + 2 * (k & 3u);
+                        umma_bf16(tmem_base + i * 128, dq + i * (tile_bytes >> 4) + off, dk + off, idesc, k != 0);
+                    }
+                umma_commit(bar_s);
+            } else {
+                // nothing may still be on its way into this CTA's shared memory when it ends
+                for (uint32_t it = 0; it < WAIT_LIMIT && !mbar_try_wait(bar, t & 1u); ++it) __nanosleep(64);
+            }
+        }
+        __syncwarp();
+        if (t < n) {
+            bool ok = mbar_wait(bar, t & 1u, s_abort, p.status) && mbar_wait(bar_s, t & 1u, s_abort, p.status);
+            ok = __all_sync(0xffffffffu, ok);
+            if (ok) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+                for (uint32_t c = 0; c < 128; c += 16) {
+                    uint32_t s[16];
+                    tmem_ld16(tmem_s + c, s);
+#pragma unroll
+                    for (int x = 0; x < 16; ++x) {
+                        // `top` is at most GROWTH below the maximum: no weight is above 1. Not fused: a large exponent's rounding cancels
+                        const float w = exp2f(__fsub_rn(__fmul_rn(__uint_as_float(s[x]), p.to_log2), top) - GROWTH);
+                        s[x] = __float_as_uint(w);
+                        if (t * 128 + c + x < limit) sum += w;
+                    }
+                    tmem_st16(tmem_s + c, s);
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+#pragma unroll 1
+                for (uint32_t g = 0; 16 * g < a.d; ++g) {
+                    if (!spoilt(g)) continue;
+                    uint32_t o[16];
+                    if (t > 0) tmem_ld16(tmem_o + 16 * g, o);
+                    float acc[16];
+#pragma unroll
+                    for (int x = 0; x < 16; ++x) acc[x] = t > 0 ? __uint_as_float(o[x]) : 0.0f;
+                    const uint8_t* values = sm + at.v + (g >> 2) * TILE_CHUNK;
+#pragma unroll 1
+                    for (uint32_t c = 0; c < 128 && t * 128 + c < seen; c += 16) {
+                        uint32_t w[16];
+                        tmem_ld16(tmem_s + c, w);
+#pragma unroll
+                        for (int x = 0; x < 16; ++x) {
+                            const uint32_t key = c + x;     // the row's 16-byte units stand at their number xor key % 8 (128-byte swizzle)
+                            const uint4* v = reinterpret_cast<const uint4*>(values + key * 128);
+                            const uint4 lo = v[(2 * (g & 3u)) ^ (key & 7u)], hi = v[(2 * (g & 3u) + 1) ^ (key & 7u)];
+                            if (t * 128 + key < limit) {
+                                const uint32_t e[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                                for (int y = 0; y < 8; ++y) {
+                                    const float2 f = widen_pair<F16>(e[y]);
+                                    acc[2 * y] = fmaf(__uint_as_float(w[x]), f.x, acc[2 * y]);
+                                    acc[2 * y + 1] = fmaf(__uint_as_float(w[x]), f.y, acc[2 * y + 1]);
+                                }
+                            }
+                        }
+                        __syncwarp();
+                    }
+#pragma unroll
+                    for (int x = 0; x < 16; ++x) o[x] = __float_as_uint(acc[x]);
+                    tmem_st16(tmem_o + 16 * g, o);
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+    if (n && !*s_abort) {
+        uint16_t* out = (uint16_t*)a.out + ((uint64_t)plane * a.m + row) * a.d;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            if (16 * g >= a.d) break;
+            if (!spoilt(g)) continue;
+            uint32_t o[16];
+            tmem_ld16(tmem_o + 16 * g, o);
+#pragma unroll
+            for (int x = 0; x < 16; ++x)
+                if (mine[g >> 1] >> (16 * (g & 1) + x) & 1u) out[16 * g + x] = holo::narrow16(__fdiv_rn(__uint_as_float(o[x]), sum), F16 ? HOLO_DTYPE_F16 : HOLO_DTYPE_BF16);
+        }
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+}
+
+template <bool F16>
 __global__ void __launch_bounds__(ROWS_WARPS * 32, 1)
 attention_rows_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ RowsParams p) {
@@ -67,13 +227,13 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* sm = smem_raw + (base - raw);
     const uint32_t tile_bytes = p.chunks * TILE_CHUNK;
-    const uint32_t s_q = base, s_k = s_q + p.nq * tile_bytes, s_v = s_k + 2 * tile_bytes;
-    const uint32_t off_bars = (p.nq + 4) * tile_bytes;
+    const RowsTail at(p.nq, tile_bytes);
+    const uint32_t s_q = base + at.q, s_k = base + at.k, s_v = base + at.v, off_bars = at.bars;
     const uint32_t bar_q = base + off_bars, bar_k_full = bar_q + 8, bar_k_empty = bar_k_full + 16, bar_v_full = bar_k_empty + 16,
                    bar_v_empty = bar_v_full + 16, bar_s = bar_v_empty + 16, bar_p = bar_s + 16, bar_pv = bar_p + 16;
-    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(sm + off_bars + 128);
-    volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(sm + off_bars + 132);
-    volatile uint32_t* s_redo = reinterpret_cast<volatile uint32_t*>(sm + off_bars + 136);
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(sm + off_bars + RowsTail::TMEM);
+    volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(sm + off_bars + RowsTail::ABORT);
+    volatile uint32_t* s_again = reinterpret_cast<volatile uint32_t*>(sm + off_bars + RowsTail::AGAIN);
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t plane = blockIdx.x, kv_plane = plane / a.h * a.hkv + plane % a.h / (a.h / a.hkv);
@@ -89,8 +249,11 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             mbar_init(bar_p + 8 * s, 4);     // one arrival per softmax warp
             mbar_init(bar_pv + 8 * s, 1);
         }
+        mbar_init(base + off_bars + RowsTail::AGAIN_BAR, 1);
+        mbar_init(base + off_bars + RowsTail::AGAIN_SCORES_BAR, 1);
         *s_abort = 0;
-        *s_redo = 0;
+        *s_again = 0;
+        *reinterpret_cast<uint4*>(sm + off_bars + RowsTail::SPOILT) = make_uint4(0, 0, 0, 0);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     holo_pdl_wait();
@@ -294,7 +457,10 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                         reinterpret_cast<uint4*>(out + c)[1] = make_uint4(w[4], w[5], w[6], w[7]);
                     }
                 }
-                if (row < a.m && !finite) *s_redo = 1;
+                // a row whose maximum is +inf is NaN throughout
+                const int what = row >= a.m || top == INFINITY ? ROW_STAYS : fabsf(top) >= WILD || !isfinite(inv) ? ROW_ALL : finite ? ROW_STAYS : ROW_COLUMNS;
+                reinterpret_cast<float2*>(sm + off_bars + RowsTail::ROWS)[threadIdx.x - 64] = make_float2(top, (float)what);
+                if (what != ROW_STAYS) *s_again = 1;
             }
         }
     }
@@ -302,16 +468,10 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*s_again && !*s_abort) compute_again<F16>(map_k, map_v, p, sm, tmem_base, row0, n0, n1);
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
-    }
-    if (*s_redo && !*s_abort) {
-        // the tiles' memory is free: every load has been waited for and every product has ended
-        for (uint32_t row = row0; row < min(row0 + p.nq * 128, a.m); ++row) {
-            holo_attn::attention_row<false, ROWS_WARPS>(a, plane * a.m + row, reinterpret_cast<float*>(sm));
-            __syncthreads();
-        }
     }
 }
 
@@ -358,7 +518,7 @@ int32_t holo_try_attention_tile(holo_b200_ctx* ctx, const HoloAttnArgs& a, bool*
     HOLO_TRY(make_rows_map(&mq, a.q, a.d, a.m, (uint32_t)planes));
     HOLO_TRY(make_rows_map(&mk, a.k_new, a.d, a.m, a.b * a.hkv));
     HOLO_TRY(make_rows_map(&mv, a.v_new, a.d, a.m, a.b * a.hkv));
-    const uint32_t smem = (p.nq + 4) * p.chunks * TILE_CHUNK + 256 + 1024;   // barriers, alignment slack
+    const uint32_t smem = (p.nq + 4) * p.chunks * TILE_CHUNK + RowsTail::BYTES + 1024;   // barriers and rows, alignment slack
     const dim3 grid((uint32_t)planes, (uint32_t)((tiles + p.nq - 1) / p.nq));
     *taken = true;
     return a.dtype == HOLO_DTYPE_F16 ? launch_rows<true>(ctx, mq, mk, mv, p, grid, smem) : launch_rows<false>(ctx, mq, mk, mv, p, grid, smem);

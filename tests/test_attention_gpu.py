@@ -469,7 +469,7 @@ def same_as_general(backend, monkeypatch, run, dtype):
     assert np.max(np.abs(got[fine] - want[fine])) <= ATTENTION_TOL[dtype] * np.max(np.abs(want[fine]))
 
 
-@pytest.mark.parametrize("dtype", [F32])
+@pytest.mark.parametrize("dtype", [F32, BF, kc.DTYPE_F16])
 @pytest.mark.parametrize("b,h,kv,s,d,causal,sigma", [(1, 4, 2, 200, 64, True, 1.0), (1, 4, 2, 131, 64, False, 6.0), (2, 3, 3, 70, 128, True, 6.0), (1, 2, 2, 300, 128, False, 1.0),
                                                      (1, 80, 4, 300, 48, True, 1.0), (1, 4, 4, 260, 80, True, 1.0)])
 def test_infinities_and_nan_reach_the_rows_that_see_them(backend, monkeypatch, dtype, b, h, kv, s, d, causal, sigma):
@@ -548,7 +548,7 @@ def test_a_few_f32_rows_take_the_quicker_route(monkeypatch, b, h, kv, s, d, caus
     assert now <= 1.15 * general, (now, general)
 
 
-@pytest.mark.parametrize("dtype", [F32])
+@pytest.mark.parametrize("dtype", [F32, BF, kc.DTYPE_F16])
 @pytest.mark.parametrize("b,h,kv,s,d,causal", [(1, 12, 12, 128, 64, True), (1, 1, 1, 128, 128, False), (1, 8, 8, 381, 64, True), (1, 32, 8, 512, 128, False)])
 def test_a_value_that_is_not_finite_costs_no_more_than_the_general_routine(monkeypatch, b, h, kv, s, d, causal, dtype):
     # every row sees it, in one column: f32, 12 heads of 128 rows took 718 us where the general routine takes 87
@@ -558,3 +558,16 @@ def test_a_value_that_is_not_finite_costs_no_more_than_the_general_routine(monke
     x.append(torch.empty_like(x[0]))
     now, general = times(kc.KernelCall.Attention(kc.AttentionCall(*[kc.rb(i) for i in range(4)], b, h, s, d, kv if kv != h else 0, int(causal), 0, dtype)), x, monkeypatch)
     assert now <= 1.15 * general, (now, general)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_large_finite_values_stay_finite(backend, d):
+    # the tiles' weights refer to a maximum that lags by up to 2^8: a value near the type's largest overflows there and is computed again
+    b, h, s = 1, 2, 300
+    q, k, v = attention_inputs(b, h, h, s, d, BF, 11, 6.0)
+    v.reshape(h, s, d)[:, ::7, 3] = orc.f32_to_bf16_rne(np.full(1, 2e37, np.float32))[0]
+    got = wide(run_attention(backend, q, k, v, b, h, h, s, d, False, BF), BF).reshape(h, s, d).astype(np.float64)
+    from helpers import attention_f64
+    want = attention_f64(wide(q, BF), wide(k, BF), wide(v, BF), b, h, h, s, d, False, None).reshape(h, s, d)
+    assert np.isfinite(got).all()
+    assert np.abs(got - want)[..., 3].max() <= 2.0 ** -7 * np.abs(want[..., 3]).max()
