@@ -379,6 +379,18 @@ def test_single_token_attention_over_a_float_cache(backend, b, h, kv, past, vali
     ws.close()
 
 
+def run_decode(backend, arrs, valid, b, h, kv, m, past, d, dtype):
+    ws = hb.DeviceWorkspace(backend, 7)
+    for i, x in enumerate(arrs):
+        ws.put(i, x)
+    ws.put(5, np.array([valid], dtype=np.uint32))
+    ws.alloc(6, arrs[0].nbytes)
+    backend.dispatch(kc.KernelCall.DecodeAttentionValid(kc.DecodeAttentionValidCall(*[kc.rb(i) for i in range(7)], b, h, kv, m, past, m, d, 0, dtype)), ws)
+    out = ws.read(6, arrs[0].nbytes, arrs[0].dtype)
+    ws.close()
+    return out
+
+
 @pytest.mark.parametrize("dtype", [F32, BF])
 def test_recorded_calls_of_one_context_share_nothing(dtype):
     # two graphs recorded from one context, replayed side by side on two streams: each gives its own call's result every time
@@ -486,6 +498,52 @@ def test_infinities_and_nan_reach_the_rows_that_see_them(backend, monkeypatch, d
     k4[b - 1, kv - 1, 17, 0] = big
     same_as_general(backend, monkeypatch, lambda: run_attention(backend, q, k, v, b, h, kv, s, d, causal, dtype), dtype)
 
+
+@pytest.mark.parametrize("dtype", [F32, BF, kc.DTYPE_F16])
+def test_one_row_sees_infinities_and_nan_of_its_cache(backend, monkeypatch, dtype):
+    # keys split over warps, a cluster and clusters: one column's infinities meet, one stays, an infinite score in the other kv head
+    b, h, kv, past, d = 1, 4, 2, 700, 64
+    rng = np.random.default_rng(13)
+    arrs = [rng.standard_normal(n).astype(np.float32) for n in (b * h * d, b * kv * past * d, b * kv * past * d, b * kv * d, b * kv * d)]
+    if dtype != F32:
+        arrs = [orc.f32_to_bf16_rne(x) if dtype == BF else x.astype(np.float16).view(np.uint16) for x in arrs]
+    inf, ninf, nan = SPECIAL[dtype]
+    arrs[0].reshape(h, d)[2:, 0] = (0x3f80, 0xbf80) if dtype == BF else (0x3c00, 0xbc00) if dtype != F32 else (1.0, -1.0)   # one row's score is +inf, the other's -inf
+    v, k = arrs[2].reshape(kv, past, d), arrs[1].reshape(kv, past, d)
+    v[0, 5, 2], v[0, 600, 2], v[0, 300, 7], arrs[4].reshape(kv, d)[0, 9] = inf, ninf, ninf, inf
+    k[1, 417, 0] = inf
+    same_as_general(backend, monkeypatch, lambda: run_decode(backend, arrs, past, b, h, kv, 1, past, d, dtype), dtype)
+
+
+# up to 64 query rows of a kv head that all see the same keys: blocks of one, four and eight rows, the last one padded
+@pytest.mark.parametrize("b,h,kv,s,d,dtype", [(1, 3, 3, 2, 64, BF), (1, 8, 2, 7, 64, kc.DTYPE_F16), (2, 12, 4, 15, 64, BF), (1, 4, 1, 15, 128, kc.DTYPE_F16), (1, 4, 2, 9, 200, BF),
+                                              (1, 5, 5, 3, 16, kc.DTYPE_F16), (1, 4, 2, 5, 160, F32), (1, 2, 1, 30, 256, F32), (3, 2, 2, 2, 132, F32)])
+def test_short_sequences_without_the_causal_law(backend, b, h, kv, s, d, dtype):
+    from helpers import attention_f64
+    q, k, v = attention_inputs(b, h, kv, s, d, dtype, s + d, 2.0)
+    got = wide(run_attention(backend, q, k, v, b, h, kv, s, d, False, dtype), dtype)
+    assert norm_max_err(got, attention_f64(wide(q, dtype), wide(k, dtype), wide(v, dtype), b, h, kv, s, d, False, None)) <= ATTENTION_TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", [BF, kc.DTYPE_F16])
+def test_weights_are_held_in_more_than_16_bits(backend, dtype):
+    # Values of +A and -A: a cell whose sum nearly cancels shows the weights' own error, which elsewhere is below the output's last bit.
+    # Unit: A times the 2-norm of the row's weights, which is at least A / 8 for 64 keys. Two bf16 terms err by at most 2^-17 of a weight,
+    # so by 2^-14 units; the output's rounding by 2^-7 of the at most 2^-6 units that are looked at: together under 2^-12. One term would
+    # err by 2^-9 of each weight, 2^-9.8 units on average. f16: 2^-14 where one term errs by 2^-12.8 on average.
+    b, h, s, d, a = 1, 8, 64, 64, 1024.0
+    q, k, v = attention_inputs(b, h, h, s, d, dtype, 21)
+    v = np.where(wide(v, dtype) > 0, a, -a).astype(np.float32)
+    stored = orc.f32_to_bf16_rne(v) if dtype == BF else v.astype(np.float16).view(np.uint16)
+    got = wide(run_attention(backend, q, k, stored, b, h, h, s, d, False, dtype), dtype).reshape(h, s, d).astype(np.float64)
+    q4, k4, v4 = (x.astype(np.float64).reshape(h, s, d) for x in (wide(q, dtype), wide(k, dtype), v))
+    e = np.einsum("hqd,hkd->hqk", q4, k4) / np.sqrt(d)
+    w = np.exp(e - e.max(-1, keepdims=True))
+    w /= w.sum(-1, keepdims=True)
+    want, unit = np.einsum("hqk,hkd->hqd", w, v4), a * np.sqrt((w * w).sum(-1, keepdims=True))
+    near = np.abs(want) <= 2.0 ** -6 * unit
+    assert near.sum() > 200
+    assert (np.abs(got - want) / unit)[near].max() <= (2.0 ** -12 if dtype == BF else 2.0 ** -14)
 
 
 # ---- routes ----
