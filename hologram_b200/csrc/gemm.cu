@@ -100,12 +100,10 @@ int32_t holo_launch_matmul_multi(holo_b200_ctx* ctx, const void* a, const void* 
     }
     if (cell_path) return holo_launch_matmul_cell(ctx, a, b, out, table, segs[0].fused_act ? lut_id_of_fused(segs[0].fused_act) : -1, residual, m, k, n, dtype, 0);
     const uint32_t kblocks = (k + BK - 1) / BK, mtiles = (m + BM - 1) / BM;
-    // Compute-bound shapes (at least one 128 x 256 tile per SM): the persistent kernel.
     {
-        bool persistent, paired;
-        persistent_choice(ctx, m, n, &persistent, &paired);
-        if (gated || (segs[0].all_reduce && ctx->tp_world > 1)) persistent = paired = false;
-        if (persistent) {
+        BigKernel big = big_choice(ctx, m, n, kblocks);
+        if (gated || (segs[0].all_reduce && ctx->tp_world > 1)) big = CTA_PER_TILE;
+        if (big != CTA_PER_TILE) {
             GemmParams p;
             memset(&p, 0, sizeof p);
             for (uint32_t i = 0; i < MAX_SEGS; ++i) p.seg[i] = gs[i];
@@ -117,8 +115,11 @@ int32_t holo_launch_matmul_multi(holo_b200_ctx* ctx, const void* a, const void* 
             CUtensorMap ma, mb;
             HOLO_TRY(make_map_2d(&ma, a, k, m, BK, BM));
             HOLO_TRY(make_map_2d(&mb, b, n, k, 64, BK));
-            if (dtype == HOLO_DTYPE_F16) return paired ? launch_pair<true, false>(ctx, ma, mb, p) : launch_persistent<true, false>(ctx, ma, mb, p);
-            return paired ? launch_pair<false, false>(ctx, ma, mb, p) : launch_persistent<false, false>(ctx, ma, mb, p);
+            if (dtype == HOLO_DTYPE_F16)
+                return big == PAIRS ? launch_pair<true, false, false>(ctx, ma, mb, p) : big == HALF_PAIRS ? launch_pair<true, false, true>(ctx, ma, mb, p)
+                                                                                                          : launch_persistent<true, false>(ctx, ma, mb, p);
+            return big == PAIRS ? launch_pair<false, false, false>(ctx, ma, mb, p) : big == HALF_PAIRS ? launch_pair<false, false, true>(ctx, ma, mb, p)
+                                                                                                       : launch_persistent<false, false>(ctx, ma, mb, p);
         }
     }
     int bn;

@@ -515,21 +515,20 @@ matmul_bf16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             constexpr uint32_t fmt = F16 ? 0u : 1u;
             const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
             bool ok = true;
+            // A: 16 k-elements = 32 bytes inside the swizzled 128-byte row; 8-row groups 1024 B apart
+            // B: 16 k-rows = two 8-row groups (1024 B apart); 64-column chunks BK*128 B apart
+            const uint64_t desc_a = smem_desc(base, 16, 1024), desc_b = smem_desc(base + S::A_BYTES, BK * 128, 1024);
+            uint32_t s = 0, phase = 0;
             for (uint32_t i = 0; i < nkb && ok; ++i) {
-                const uint32_t s = i % STAGES, use = i / STAGES;
-                ok = mbar_wait(bar_full + 8 * s, use & 1, s_abort, p.status);
+                ok = mbar_wait(bar_full + 8 * s, phase, s_abort, p.status);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a_addr = base + s * S::STAGE, b_addr = a_addr + S::A_BYTES;
+                const uint64_t da = desc_a + s * (S::STAGE >> 4), db = desc_b + s * (S::STAGE >> 4);
+                umma_bf16(tmem_base, da, db, idesc, i != 0 ? 1u : 0u);
 #pragma unroll
-                for (int j = 0; j < BK / 16; ++j) {
-                    // A: 16 k-elements = 32 bytes inside the swizzled 128-byte row; 8-row groups 1024 B apart
-                    const uint64_t da = smem_desc(a_addr + j * 32, 16, 1024);
-                    // B: 16 k-rows = two 8-row groups (1024 B apart); 64-column chunks BK*128 B apart
-                    const uint64_t db = smem_desc(b_addr + j * 2048, BK * 128, 1024);
-                    umma_bf16(tmem_base, da, db, idesc, (i | (uint32_t)j) != 0 ? 1u : 0u);
-                }
+                for (int j = 1; j < BK / 16; ++j) umma_bf16(tmem_base, da + 2 * j, db + 128 * j, idesc, 1u);
                 umma_commit(bar_empty + 8 * s);  // frees the ring slot once these MMAs have read it
+                if (++s == STAGES) s = 0, phase ^= 1u;
             }
             if (ok && nkb != 0) umma_commit(bar_accum);      // accumulator complete
         }
@@ -931,7 +930,7 @@ matmul_umma_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const _
         if (lane == 0) {
             const uint32_t tx = S::A_BYTES + S::B_BYTES;
             const uint32_t a_start = LIN && p.a_pos ? lin_a_start(p) : 0u;
-            uint32_t it = 0;
+            uint32_t s = 0, phase = 1;      // the first round of the ring finds its slots free
             bool ok = true;
             for (uint32_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
                 const int m0 = (int)((tile / tiles_n) * BM), n0 = (int)((tile % tiles_n) * PBN);
@@ -941,15 +940,15 @@ matmul_umma_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const _
                     const LinTile t = lin_tile(p, a_start, tile / tiles_n, (uint32_t)m0);
                     a_row = (int)t.a_row; b_row = (int)t.b_row;
                 }
-                for (uint32_t kb = 0; kb < p.kblocks; ++kb, ++it) {
-                    const uint32_t s = it % PSTAGES, use = it / PSTAGES;
-                    if (use > 0 && !mbar_wait(bar_empty + 8 * s, (use - 1) & 1, s_abort, p.status)) { ok = false; break; }
+                for (uint32_t kb = 0; kb < p.kblocks; ++kb) {
+                    if (!mbar_wait(bar_empty + 8 * s, phase, s_abort, p.status)) { ok = false; break; }
                     const uint32_t st = base + s * S::STAGE;
                     const int k0 = (int)(kb * BK);
                     mbar_arrive_expect_tx(bar_full + 8 * s, tx);
                     tma_load_2d(st, &map_a, k0 + a_k0, a_row, bar_full + 8 * s);
 #pragma unroll
                     for (int h = 0; h < PBN / 64; ++h) tma_load_2d(st + S::A_BYTES + h * (BK * 128), &map_b, n0 + 64 * h, k0 + b_row, bar_full + 8 * s);
+                    if (++s == PSTAGES) s = 0, phase ^= 1u;
                 }
             }
         }
@@ -958,7 +957,8 @@ matmul_umma_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const _
         if (lane == 0) {
             constexpr uint32_t fmt = F16 ? 0u : 1u;
             const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 16) | ((uint32_t)(PBN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-            uint32_t it = 0, t = 0;
+            const uint64_t desc_a = smem_desc(base, 16, 1024), desc_b = smem_desc(base + S::A_BYTES, BK * 128, 1024);
+            uint32_t s = 0, phase = 0, t = 0;
             bool ok = true;
             for (uint32_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++t) {
                 const uint32_t buf = t & 1u, use = t >> 1;
@@ -966,18 +966,15 @@ matmul_umma_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const _
                 if (use > 0 && !mbar_wait(bar_acc_empty + 8 * buf, (use - 1) & 1, s_abort, p.status)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t tmem_d = tmem_base + buf * (uint32_t)PBN;
-                for (uint32_t kb = 0; kb < p.kblocks; ++kb, ++it) {
-                    const uint32_t s = it % PSTAGES;
-                    if (!mbar_wait(bar_full + 8 * s, (it / PSTAGES) & 1, s_abort, p.status)) { ok = false; break; }
+                for (uint32_t kb = 0; kb < p.kblocks; ++kb) {
+                    if (!mbar_wait(bar_full + 8 * s, phase, s_abort, p.status)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a_addr = base + s * S::STAGE, b_addr = a_addr + S::A_BYTES;
+                    const uint64_t da = desc_a + s * (S::STAGE >> 4), db = desc_b + s * (S::STAGE >> 4);
+                    umma_bf16(tmem_d, da, db, idesc, kb != 0 ? 1u : 0u);
 #pragma unroll
-                    for (int j = 0; j < BK / 16; ++j) {
-                        const uint64_t da = smem_desc(a_addr + j * 32, 16, 1024);
-                        const uint64_t db = smem_desc(b_addr + j * 2048, BK * 128, 1024);
-                        umma_bf16(tmem_d, da, db, idesc, (kb | (uint32_t)j) != 0 ? 1u : 0u);
-                    }
+                    for (int j = 1; j < BK / 16; ++j) umma_bf16(tmem_d, da + 2 * j, db + 128 * j, idesc, 1u);
                     umma_commit(bar_empty + 8 * s);
+                    if (++s == PSTAGES) s = 0, phase ^= 1u;
                 }
                 if (ok) umma_commit(bar_acc_full + 8 * buf);
             }
@@ -1054,15 +1051,17 @@ matmul_umma_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const _
 //   both CTAs  warp 0: TMA producer for its halves (waits on its own "empty" barriers, signals the leader's "full")
 //   leader     warp 1: MMA issuer; tcgen05.commit multicasts "slot free" and "accumulator ready" to both CTAs
 //   both CTAs  warps 2-5: epilogue from their own TMEM; hand the TMEM half back by arriving on the leader's barrier
-// The accumulator is double-buffered (2 x 256 columns), the ring has 7 stages and never drains between tiles.
+// The accumulator is double-buffered (2 x 256 columns); the ring never drains between tiles. It has three stages of two k-blocks (three
+// where every item is 256 x 128): what one stage costs in waits, commits and barriers across the pair is paid once for them.
 // Every mbarrier wait is bounded; the only unbounded waits are the two cluster barriers (after barrier set-up
 // and before TMEM is released), which every thread of both CTAs reaches after bounded waits only.
-constexpr int QSTAGES = 7;
+constexpr int QSTAGES = 3;
+template <bool HALVES>
 struct PairSmem {
-    static constexpr uint32_t A_BYTES = BM * BK * 2;            // this CTA's 128 rows: 16 KiB
-    static constexpr uint32_t B_BYTES = BK * 128 * 2;           // this CTA's 128 columns: 16 KiB
-    static constexpr uint32_t STAGE = A_BYTES + B_BYTES;
-    static constexpr uint32_t RING = QSTAGES * STAGE;           // 224 KiB: what arrives from L2 takes 1-2 us, so every KiB in flight counts
+    static constexpr uint32_t A_BYTES = BM * BK * 2;                        // this CTA's 128 rows: 16 KiB
+    static constexpr uint32_t B_BYTES = BK * (HALVES ? 64 : 128) * 2;       // this CTA's columns: 8 or 16 KiB
+    static constexpr uint32_t BLOCK = A_BYTES + B_BYTES, BLOCKS = HALVES ? 3 : 2, STAGE = BLOCKS * BLOCK;
+    static constexpr uint32_t RING = QSTAGES * STAGE;                       // 216 or 192 KiB
     static constexpr uint32_t TOTAL = RING + 256 + 1024;
 };
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t cta_rank) {
@@ -1076,10 +1075,11 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(leader_bar)
         : "memory");
 }
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint32_t a_low, uint32_t a_high, uint32_t b_low, uint32_t b_high, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        "{\n.reg .pred p;\n.reg .b64 a, b;\nmov.b64 a, {%1, %2};\nmov.b64 b, {%3, %4};\nsetp.ne.b32 p, %6, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %5, p;\n}\n"
+        ::"r"(tmem_d), "r"(a_low), "r"(a_high), "r"(b_low), "r"(b_high), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // arrive on the barrier at this offset in both CTAs of the pair once the MMAs issued so far have completed
@@ -1092,9 +1092,15 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
 struct PairItem {
     uint32_t m_tile, n0, bn;
 };
+template <bool HALVES>
 __device__ __forceinline__ PairItem pair_item(const GemmParams& p, uint32_t w, uint32_t tiles_n) {
     PairItem it;
-    if (w < p.tail_begin) {
+    if (HALVES) {
+        const uint32_t across = (p.n + 127) / 128;
+        it.m_tile = w / across;
+        it.n0 = (w % across) * 128;
+        it.bn = 128;
+    } else if (w < p.tail_begin) {
         it.m_tile = w / tiles_n;
         it.n0 = (w % tiles_n) * 256;
         it.bn = 256;
@@ -1107,10 +1113,11 @@ __device__ __forceinline__ PairItem pair_item(const GemmParams& p, uint32_t w, u
     return it;
 }
 
-template <bool F16, bool LIN>
+// HALVES: every item is 256 x 128.
+template <bool F16, bool LIN, bool HALVES>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 matmul_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
-    using S = PairSmem;
+    using S = PairSmem<HALVES>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -1123,7 +1130,7 @@ matmul_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // the pair is a cluster of two along grid x (the hardware pairs CTAs whose cluster rank differs in the lowest bit)
     const uint32_t rank = blockIdx.x & 1u, pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;   // rank 0 = leader
-    const uint32_t tiles_n = (p.n + 255) / 256, tiles_m = (p.m + 255) / 256, ntiles = tiles_n * tiles_m;
+    const uint32_t tiles_n = (p.n + 255) / 256;
 
     holo_pdl_trigger();
     if (threadIdx.x == 0) {
@@ -1156,25 +1163,29 @@ matmul_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         // ---------------- TMA producer (both CTAs) ----------------
         if (lane == 0) {
             const uint32_t a_start = LIN && p.a_pos ? lin_a_start(p) : 0u;
-            uint32_t it = 0;
+            const uint32_t leader_full = map_to_cta(bar_full, 0);
+            uint32_t s = 0, phase = 1;      // the first round of the ring finds its slots free
             bool ok = true;
             for (uint32_t w = pair; w < p.n_items && ok; w += npairs) {
-                const PairItem item = pair_item(p, w, tiles_n);
+                const PairItem item = pair_item<HALVES>(p, w, tiles_n);
                 // this CTA's halves: rows [128 r, +128) of the A block, columns [bn/2 r, +bn/2) of the B block
                 const int m0 = (int)(item.m_tile * 256 + rank * 128), n0 = (int)(item.n0 + rank * (item.bn >> 1));
                 const int a_k0 = LIN ? (int)p.lin[lin_segment(p, item.n0)].k_offset : 0;
                 const int a_row = LIN && p.a_pos ? (int)lin_a_row(p, a_start, (uint32_t)m0) : m0;
                 const uint32_t tx = 2u * (S::A_BYTES + (item.bn >> 1) * BK * 2);
-                for (uint32_t kb = 0; kb < p.kblocks; ++kb, ++it) {
-                    const uint32_t s = it % QSTAGES, use = it / QSTAGES;
-                    if (use > 0 && !mbar_wait(bar_empty + 8 * s, (use - 1) & 1, s_abort, p.status)) { ok = false; break; }
-                    const uint32_t st = base + s * S::STAGE;
-                    const int k0 = (int)(kb * BK);
-                    if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * s, tx);
-                    const uint32_t leader_bar = map_to_cta(bar_full + 8 * s, 0);
-                    tma_load_2d_pair(st, &map_a, k0 + a_k0, a_row, leader_bar);
-                    tma_load_2d_pair(st + S::A_BYTES, &map_b, n0, k0, leader_bar);
-                    if (item.bn == 256) tma_load_2d_pair(st + S::A_BYTES + BK * 128, &map_b, n0 + 64, k0, leader_bar);
+                for (uint32_t kb = 0; kb < p.kblocks; kb += S::BLOCKS) {
+                    if (!mbar_wait(bar_empty + 8 * s, phase, s_abort, p.status)) { ok = false; break; }
+                    const uint32_t st = base + s * S::STAGE, left = p.kblocks - kb, leader_bar = leader_full + 8 * s;
+                    if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * s, tx * min(left, S::BLOCKS));
+#pragma unroll
+                    for (uint32_t i = 0; i < S::BLOCKS; ++i) {
+                        if (i >= left) break;
+                        const int k0 = (int)((kb + i) * BK);
+                        tma_load_2d_pair(st + i * S::BLOCK, &map_a, k0 + a_k0, a_row, leader_bar);
+                        tma_load_2d_pair(st + i * S::BLOCK + S::A_BYTES, &map_b, n0, k0, leader_bar);
+                        if (!HALVES && item.bn == 256) tma_load_2d_pair(st + i * S::BLOCK + S::A_BYTES + BK * 128, &map_b, n0 + 64, k0, leader_bar);
+                    }
+                    if (++s == QSTAGES) s = 0, phase ^= 1u;
                 }
             }
         }
@@ -1184,26 +1195,30 @@ matmul_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             constexpr uint32_t fmt = F16 ? 0u : 1u;
             // D = f32, A = B = bf16 / f16, A K-major, B N-major, N = 256 (128 for a tail half), M = 256 (128 rows in each CTA)
             const uint32_t idesc_base = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 16) | ((uint32_t)(256 >> 4) << 24);
-            uint32_t it = 0, t = 0;
+            // descriptors in two words: steps only change the lower one
+            const uint64_t first_a = smem_desc(base, 16, 1024), first_b = smem_desc(base + S::A_BYTES, BK * 128, 1024);
+            const uint32_t desc_a = (uint32_t)first_a, high_a = (uint32_t)(first_a >> 32), desc_b = (uint32_t)first_b, high_b = (uint32_t)(first_b >> 32);
+            uint32_t s = 0, phase = 0, t = 0;
             bool ok = true;
             for (uint32_t w = pair; w < p.n_items && ok; w += npairs, ++t) {
-                const uint32_t idesc = idesc_base | ((pair_item(p, w, tiles_n).bn >> 3) << 17);
+                const uint32_t idesc = idesc_base | ((pair_item<HALVES>(p, w, tiles_n).bn >> 3) << 17);
                 const uint32_t buf = t & 1u, use = t >> 1;
                 if (use > 0 && !mbar_wait(bar_acc_empty + 8 * buf, (use - 1) & 1, s_abort, p.status)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t tmem_d = tmem_base + buf * 256u;
-                for (uint32_t kb = 0; kb < p.kblocks; ++kb, ++it) {
-                    const uint32_t s = it % QSTAGES;
-                    if (!mbar_wait(bar_full + 8 * s, (it / QSTAGES) & 1, s_abort, p.status)) { ok = false; break; }
+                for (uint32_t kb = 0; kb < p.kblocks; kb += S::BLOCKS) {
+                    if (!mbar_wait(bar_full + 8 * s, phase, s_abort, p.status)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a_addr = base + s * S::STAGE, b_addr = a_addr + S::A_BYTES;
+                    const uint32_t left = p.kblocks - kb, da = desc_a + s * (S::STAGE >> 4), db = desc_b + s * (S::STAGE >> 4);
 #pragma unroll
-                    for (int j = 0; j < BK / 16; ++j) {
-                        const uint64_t da = smem_desc(a_addr + j * 32, 16, 1024);
-                        const uint64_t db = smem_desc(b_addr + j * 2048, BK * 128, 1024);
-                        umma_bf16_pair(tmem_d, da, db, idesc, (kb | (uint32_t)j) != 0 ? 1u : 0u);
+                    for (uint32_t i = 0; i < S::BLOCKS; ++i) {
+                        if (i >= left) break;
+#pragma unroll
+                        for (uint32_t j = 0; j < BK / 16; ++j)
+                            umma_bf16_pair(tmem_d, da + i * (S::BLOCK >> 4) + 2 * j, high_a, db + i * (S::BLOCK >> 4) + 128 * j, high_b, idesc, i + j != 0 || kb != 0 ? 1u : 0u);
                     }
                     umma_commit_pair(bar_empty + 8 * s);
+                    if (++s == QSTAGES) s = 0, phase ^= 1u;
                 }
                 if (ok) umma_commit_pair(bar_acc_full + 8 * buf);
             }
@@ -1217,7 +1232,7 @@ matmul_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         uint32_t t = 0;
         for (uint32_t w = pair; w < p.n_items; w += npairs, ++t) {
             const uint32_t buf = t & 1u, use = t >> 1;
-            const PairItem item = pair_item(p, w, tiles_n);
+            const PairItem item = pair_item<HALVES>(p, w, tiles_n);
             const uint32_t m0 = item.m_tile * 256 + rank * 128, n0 = item.n0;
             const uint32_t row = m0 + quarter * 32 + lane;
             const bool got = mbar_wait(bar_acc_full + 8 * buf, use & 1, s_abort, p.status);
@@ -1332,17 +1347,17 @@ int32_t launch_umma(holo_b200_ctx* ctx, const CUtensorMap& ma, const CUtensorMap
 
 // Set the pair kernel up on this device and return how many pairs it can hold at once (a GPC with an odd number of
 // SMs leaves one unpaired).
-template <bool F16, bool LIN>
+template <bool F16, bool LIN, bool HALVES>
 int32_t pair_kernel_slots(holo_b200_ctx* ctx, uint32_t* out) {
     static thread_local int configured = -1;
     static thread_local int resident = 0;
     if (configured != ctx->device) {
         const uint32_t pairs = (uint32_t)ctx->sm_count / 2;
-        HOLO_CUDA(cudaFuncSetAttribute(matmul_umma_pair_kernel<F16, LIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::TOTAL));
+        HOLO_CUDA(cudaFuncSetAttribute(matmul_umma_pair_kernel<F16, LIN, HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<HALVES>::TOTAL));
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(2 * pairs, 1, 1);
         cfg.blockDim = dim3(GEMM_THREADS);
-        cfg.dynamicSmemBytes = PairSmem::TOTAL;
+        cfg.dynamicSmemBytes = PairSmem<HALVES>::TOTAL;
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeClusterDimension;
         at.val.clusterDim.x = 2;
@@ -1351,7 +1366,7 @@ int32_t pair_kernel_slots(holo_b200_ctx* ctx, uint32_t* out) {
         cfg.attrs = &at;
         cfg.numAttrs = 1;
         int nclusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&nclusters, matmul_umma_pair_kernel<F16, LIN>, &cfg) != cudaSuccess || nclusters <= 0) {
+        if (cudaOccupancyMaxActiveClusters(&nclusters, matmul_umma_pair_kernel<F16, LIN, HALVES>, &cfg) != cudaSuccess || nclusters <= 0) {
             cudaGetLastError();
             nclusters = (int)pairs;
         }
@@ -1364,20 +1379,20 @@ int32_t pair_kernel_slots(holo_b200_ctx* ctx, uint32_t* out) {
 
 // 256 x 256 tiles on CTA pairs. The last, partial round: when its tiles cut in two still fit one round, they run as
 // 256 x 128 halves (every pair busy for half a tile's time instead of some pairs for a whole one). Same k order per cell.
-template <bool F16, bool LIN>
+template <bool F16, bool LIN, bool HALVES>
 int32_t launch_pair(holo_b200_ctx* ctx, const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p) {
-    const uint32_t qtiles = ((p.m + 255) / 256) * ((p.n + 255) / 256), pairs = (uint32_t)ctx->sm_count / 2;
+    const uint32_t qtiles = ((p.m + 255) / 256) * (HALVES ? (p.n + 127) / 128 : (p.n + 255) / 256), pairs = (uint32_t)ctx->sm_count / 2;
     uint32_t resident;
-    HOLO_TRY((pair_kernel_slots<F16, LIN>(ctx, &resident)));
+    HOLO_TRY((pair_kernel_slots<F16, LIN, HALVES>(ctx, &resident)));
     uint32_t grid = qtiles < pairs ? qtiles : pairs;
     if (grid > resident) grid = resident;
     if (const char* e = getenv("HOLO_GEMM_PAIR_GRID")) grid = (uint32_t)atoi(e) > 0 ? (uint32_t)atoi(e) : grid;
     const uint32_t rest = qtiles % grid;
-    const bool split_tail = rest != 0 && 2 * rest <= grid && !getenv("HOLO_GEMM_NO_TAIL_SPLIT");
+    const bool split_tail = !HALVES && rest != 0 && 2 * rest <= grid && !getenv("HOLO_GEMM_NO_TAIL_SPLIT");
     p.tail_begin = split_tail ? qtiles - rest : qtiles;
     p.n_items = split_tail ? qtiles + rest : qtiles;
     // the two CTAs of a pair are a cluster along grid x
-    HOLO_CUDA(holo_launch_kernel_cluster(ctx, matmul_umma_pair_kernel<F16, LIN>, dim3(2 * grid), dim3(GEMM_THREADS), PairSmem::TOTAL, 2u, 1u, ma, mb, p));
+    HOLO_CUDA(holo_launch_kernel_cluster(ctx, matmul_umma_pair_kernel<F16, LIN, HALVES>, dim3(2 * grid), dim3(GEMM_THREADS), PairSmem<HALVES>::TOTAL, 2u, 1u, ma, mb, p));
     ctx->launches++;
     return HOLO_OK;
 }
@@ -1396,15 +1411,41 @@ int32_t launch_persistent(holo_b200_ctx* ctx, const CUtensorMap& ma, const CUten
     return HOLO_OK;
 }
 
-// Does a product with this many row tiles take the persistent kernels (at least one 128 x 256 tile per SM), and of those
-// the pair kernel (at least one 256 x 256 tile per pair of SMs)?
-inline void persistent_choice(const holo_b200_ctx* ctx, uint32_t m, uint32_t n, bool* persistent, bool* paired) {
-    const uint32_t mtiles = (m + BM - 1) / BM, ptiles = mtiles * ((n + PBN - 1) / PBN);
-    *persistent = mtiles >= 2 && ptiles >= (uint32_t)ctx->sm_count;
-    if (const char* e = getenv("HOLO_GEMM_PERSISTENT")) *persistent = *persistent && atoi(e) != 0;
-    const uint32_t qtiles = ((m + 255) / 256) * ((n + 255) / 256);
-    *paired = *persistent && qtiles >= (uint32_t)ctx->sm_count / 2;
-    if (const char* e = getenv("HOLO_GEMM_PAIR")) *paired = *paired && atoi(e) != 0;
+// Which kernel takes a product of two row tiles or more: CTA pairs on 256 x 256 tiles (PAIRS), on 256 x 128 (HALF_PAIRS), 128 x 256 tiles
+// walked by one CTA per SM (WALK), or a CTA per tile (tile_choice). What each takes, in ns, fitted to 249 shapes of 130 .. 4096 rows, each
+// timed with all four: a start and, per round of items, an epilogue and what a k-block costs. Per SM and k-block a pair reads 32 KiB for
+// 256 x 256 and 24 KiB for 256 x 128, CTAs with 128 x 64 tiles read 24 KiB each, two of them on an SM: that is why few tiles of a
+// long k do better as halves on pairs (1024 x 8192 x 2048 43.7 -> 36.5 us, 446 x 2536 x 3440 31 -> 20, 1024 x 2048 x 2048 15.5 -> 14.8), and one
+// round of whole tiles better than two of CTAs (2048 x 10240 x 2048 75 -> 63). The choice was 1 % above the best of the four on average
+// (12.9 us, geometric mean; without halves and with pairs from a full round on only, 13.5); 1.15 where the estimate misled it, hence the margins.
+enum BigKernel { CTA_PER_TILE, WALK, PAIRS, HALF_PAIRS };
+inline BigKernel big_choice(const holo_b200_ctx* ctx, uint32_t m, uint32_t n, uint32_t kblocks) {
+    const uint64_t sms = (uint64_t)ctx->sm_count, pairs = sms / 2, kb = kblocks;
+    const uint64_t mtiles = (m + BM - 1) / BM, ptiles = mtiles * ((n + PBN - 1) / PBN), quads = (uint64_t)((m + 255) / 256) * ((n + 255) / 256);
+    const uint64_t halves = (uint64_t)((m + 255) / 256) * ((n + 127) / 128);
+    if (mtiles < 2) return CTA_PER_TILE;
+    auto up = [](uint64_t a, uint64_t b) { return (a + b - 1) / b; };
+    const uint64_t grid = quads < pairs ? quads : pairs, rest = quads % grid;      // the last round's tiles run as halves where those fit one round
+    const uint64_t tenths = quads / grid * 10 + (rest == 0 ? 0 : 2 * rest <= grid ? 6 : 10);
+    const uint64_t whole_ns = 4500 + tenths * (3700 + 340 * kb) / 10, half_ns = 5200 + up(halves, pairs) * (1600 + 235 * kb);
+    BigKernel best = CTA_PER_TILE;
+    uint64_t best_ns;
+    if (ptiles >= sms && quads >= pairs) {
+        best = PAIRS;
+        best_ns = whole_ns * 17 / 20;
+    } else if (ptiles >= sms) {
+        best = WALK;
+        best_ns = 2700 + up(ptiles, sms) * (4250 + 366 * kb);
+    } else {
+        const uint64_t tiles128 = mtiles * ((n + 127) / 128), tiles64 = mtiles * ((n + 63) / 64);
+        best_ns = tiles128 < sms && tiles64 <= 2 * sms ? 5500 + (tiles64 <= sms ? 290 : 350) * kb : 6500 + up(tiles128, 2 * sms) * 480 * kb;
+    }
+    if (const char* e = getenv("HOLO_GEMM_PERSISTENT"))
+        if (atoi(e) == 0) return CTA_PER_TILE;
+    if (const char* e = getenv("HOLO_GEMM_PAIR"))
+        if (atoi(e) == 0) return ptiles >= sms ? WALK : CTA_PER_TILE;
+    if (best != PAIRS && whole_ns < best_ns) best = PAIRS, best_ns = whole_ns;
+    return half_ns < best_ns ? HALF_PAIRS : best;
 }
 
 // Tile width and K split of the one-tile-per-CTA kernel. Compute-bound shapes (many row tiles) take 128-wide tiles, no split.

@@ -219,16 +219,17 @@ int32_t holo_launch_linear(holo_b200_ctx* ctx, const HoloLinearArgs& a) {
     HOLO_TRY(make_map_2d(&mb, a.b, a.n, (uint64_t)a.k * (a.tiles ? a.experts : 1), 64, BK));
     // rows A has: the matrix's own, a ring's, or the ones all tiles of a group share
     const uint64_t a_rows = a.a_pos ? a.a_rows : a.a_shared ? a.a_shared : a.m;
-    bool persistent, paired;
-    persistent_choice(ctx, a.m, a.n, &persistent, &paired);
-    if (a.tiles) {
-        persistent = persistent && a.tile_rows == (uint32_t)BM && !a.a_shared;
-        paired = false;      // neighbouring row tiles may belong to different experts
+    BigKernel big = big_choice(ctx, a.m, a.n, kblocks);
+    if (a.tiles) {      // neighbouring row tiles may belong to different experts: no pairs
+        const bool walk = a.tile_rows == (uint32_t)BM && !a.a_shared && (uint64_t)mtiles * ((a.n + PBN - 1) / PBN) >= (uint64_t)ctx->sm_count;
+        const char* e = getenv("HOLO_GEMM_PERSISTENT");
+        big = walk && mtiles >= 2 && !(e && atoi(e) == 0) ? WALK : CTA_PER_TILE;
     }
-    if (persistent) {
+    if (big != CTA_PER_TILE) {
         p.box_m = BM;
         HOLO_TRY(make_map_2d(&ma, a.a, a.lda, a_rows, BK, BM));
-        return paired ? launch_pair<false, true>(ctx, ma, mb, p) : launch_persistent<false, true>(ctx, ma, mb, p);
+        return big == PAIRS ? launch_pair<false, true, false>(ctx, ma, mb, p) : big == HALF_PAIRS ? launch_pair<false, true, true>(ctx, ma, mb, p)
+                                                                                                  : launch_persistent<false, true>(ctx, ma, mb, p);
     }
     int bn;
     uint32_t splits;

@@ -298,3 +298,17 @@ def test_persistent_tile_kernels_within_tolerance(backend, monkeypatch, m, k, n,
         assert err <= 1e-2, (mode, err)
     backend.synchronize()
     assert np.array_equal(outs["pair"], outs["classic"]) and np.array_equal(outs["persistent"], outs["classic"])
+
+
+@pytest.mark.parametrize("m,k,n,act,res", [(257, 4160, 392, 0, False), (1000, 2544, 1936, kc.FUSED_SILU, False), (130, 8000, 264, 0, True), (300, 2000, 136, 0, False),
+                                           (300, 2056, 136, 0, False), (300, 2120, 136, 0, False), (260, 1536, 2056, 0, False), (513, 1984, 640, 0, True)])
+def test_few_row_tiles_of_a_long_k_on_half_width_pairs(backend, monkeypatch, m, k, n, act, res):
+    # fewer tiles than pairs of SMs: 256 x 128 items, three k-blocks a stage (remainders of 0, 1 and 2 among these), ragged last tiles.
+    # The tolerance is the other tensor-core kernels'; the k order per cell is theirs, so the bits are too.
+    a, b = synth(m, k, n, m + n)
+    r = orc.f32_to_bf16_rne(np.random.default_rng(1).standard_normal(m * n, dtype=np.float32)) if res else None
+    got = run(backend, a, b, m, k, n, act=act, residual=r)
+    want = orc.bf16_to_f32(orc.matmul(a, b, m, k, n, BF, act=act, residual=r))
+    assert norm_max_err(orc.bf16_to_f32(got), want) <= 1e-2
+    monkeypatch.setenv("HOLO_GEMM_PERSISTENT", "0")
+    assert np.array_equal(got, run(backend, a, b, m, k, n, act=act, residual=r))
