@@ -62,6 +62,21 @@ __device__ __forceinline__ float2 widen_pair(uint32_t v) {
     return F16 ? widen_f16(v) : make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
 }
 
+// The products with descriptors in two words: steps of a tile only change the lower one, by constants, and the one thread that issues
+// them has little time for each.
+__device__ __forceinline__ void product_ss(uint32_t tmem_d, uint32_t a, uint32_t a_high, uint32_t b, uint32_t b_high, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\n.reg .b64 x, y;\nmov.b64 x, {%1, %2};\nmov.b64 y, {%3, %4};\nsetp.ne.b32 p, %6, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %5, p;\n}\n"
+        ::"r"(tmem_d), "r"(a), "r"(a_high), "r"(b), "r"(b_high), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void product_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b, uint32_t b_high, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\n.reg .b64 y;\nmov.b64 y, {%2, %3};\nsetp.ne.b32 p, %5, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], y, %4, p;\n}\n"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b), "r"(b_high), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
 // Shared memory behind the tiles: barriers from `bars` on, flags, then what a row's weights refer to and what is to be computed again of it
 struct RowsTail {
     uint32_t q, k, v, bars;     // offsets
@@ -310,14 +325,23 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             const uint32_t type = F16 ? 0u : (1u << 7) | (1u << 10);
             const uint32_t idesc_s = (1u << 4) | type | ((128u >> 3) << 17) | ((128u >> 4) << 24);
             const uint32_t idesc_o = (1u << 4) | type | (1u << 16) | ((a.d >> 3) << 17) | ((128u >> 4) << 24);
-            const uint64_t desc_q = smem_desc(s_q, 16, 1024), desc_k = smem_desc(s_k, 16, 1024), desc_v = smem_desc(s_v, TILE_CHUNK, 1024);
+            const uint64_t first_q = smem_desc(s_q, 16, 1024), first_v = smem_desc(s_v, TILE_CHUNK, 1024);
+            const uint32_t desc_q = (uint32_t)first_q, desc_k = (uint32_t)smem_desc(s_k, 16, 1024), high_s = (uint32_t)(first_q >> 32);
+            const uint32_t desc_v = (uint32_t)first_v, high_v = (uint32_t)(first_v >> 32);
             const uint32_t step = tile_bytes >> 4, ksteps = a.d / 16;
             auto scores = [&](uint32_t q, uint32_t t) {
-                const uint64_t dq = desc_q + q * step, dk = desc_k + (t & 1u) * step;
-                const uint32_t d = tmem_base + q * 128;
-                for (uint32_t k = 0; k < ksteps; ++k) {
-                    const uint32_t off = (k >> 2) * (TILE_CHUNK >> 4) + 2 * (k & 3u);
-                    umma_bf16(d, dq + off, dk + off, idesc_s, k != 0);
+                const uint32_t dq = desc_q + q * step, dk = desc_k + (t & 1u) * step, d = tmem_base + q * 128;
+                if (t == 0) {       // in a loop: the first tile is all of a short call, for which the steps below are code to fetch
+                    for (uint32_t k = 0; k < ksteps; ++k) {
+                        const uint32_t off = (k >> 2) * (TILE_CHUNK >> 4) + 2 * (k & 3u);
+                        product_ss(d, dq + off, high_s, dk + off, high_s, idesc_s, k != 0);
+                    }
+                } else {
+#pragma unroll
+                    for (uint32_t k = 0; k < 8; ++k) {
+                        const uint32_t off = (k >> 2) * (TILE_CHUNK >> 4) + 2 * (k & 3u);
+                        if (k < ksteps) product_ss(d, dq + off, high_s, dk + off, high_s, idesc_s, k != 0);
+                    }
                 }
                 umma_commit(bar_s + 8 * q);
             };
@@ -341,16 +365,17 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     // keys past the last one any row of the tile sees have no weight: whole steps of them are left out
                     const uint32_t steps = min(8u, (keys_of(q) - t * 128 + 15) / 16);
                     const uint32_t tmem_p = tmem_base + q * 128, d = tmem_base + 256 + q * 128;
-                    const uint64_t dv = desc_v + s * step;
-                    for (uint32_t k = 0; k < steps; ++k) umma_bf16_ts(d, tmem_p + k * 8, dv + 128 * k, idesc_o, (t | k) != 0);
-                    for (uint32_t k = 0; k < steps; ++k) umma_bf16_ts(d, tmem_p + 64 + k * 8, dv + 128 * k, idesc_o, 1);
-                    umma_commit(bar_pv + 8 * q);
-                    if (next < n) {     // the next scores go where the weights are: their product first
-                        ok = mbar_wait(bar_pv + 8 * q, t & 1u, s_abort, p.status);
-                        if (!ok) break;
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        scores(q, next);
+                    const uint32_t dv = desc_v + s * step;
+                    if (steps == 8) {
+#pragma unroll
+                        for (uint32_t k = 0; k < 16; ++k) product_ts(d, tmem_p + k * 8, dv + 128 * (k & 7u), high_v, idesc_o, (k | t) != 0);
+                    } else {
+                        for (uint32_t k = 0; k < steps; ++k) product_ts(d, tmem_p + k * 8, dv + 128 * k, high_v, idesc_o, (k | t) != 0);
+                        for (uint32_t k = 0; k < steps; ++k) product_ts(d, tmem_p + 64 + k * 8, dv + 128 * k, high_v, idesc_o, 1);
                     }
+                    umma_commit(bar_pv + 8 * q);
+                    // the next scores go where the weights are; one thread's products execute in order, so nothing waits for the last one
+                    if (next < n) scores(q, next);
                 }
                 if (!ok) break;
                 umma_commit(bar_v_empty + 8 * s);
@@ -396,7 +421,7 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 const float f = grows ? ex2(top - here) : 1.0f;      // 0 from the first scores on
                 if (grows) top = here;
                 sum *= f;
-                if (t > 0) {    // this tile's scores were issued after the last product had ended: O is at rest
+                if (t > 0) {    // the barrier of this tile's scores stands for the product before them too: O is at rest
                     const uint64_t f2 = pair(f, f);
                     for (uint32_t c = 0; c < a.d; c += 16) {
                         uint32_t o[16];
