@@ -72,6 +72,21 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
         ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
         : "memory");
 }
+// The same products with descriptors in two words: steps of a tile only change the lower one, by constants, and the one thread that issues
+// them has little time for each.
+__device__ __forceinline__ void product_ss(uint32_t tmem_d, uint32_t a, uint32_t a_high, uint32_t b, uint32_t b_high, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\n.reg .b64 x, y;\nmov.b64 x, {%1, %2};\nmov.b64 y, {%3, %4};\nsetp.ne.b32 p, %6, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %5, p;\n}\n"
+        ::"r"(tmem_d), "r"(a), "r"(a_high), "r"(b), "r"(b_high), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void product_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b, uint32_t b_high, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\n.reg .b64 y;\nmov.b64 y, {%2, %3};\nsetp.ne.b32 p, %5, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], y, %4, p;\n}\n"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b), "r"(b_high), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
 // A operand (128 x 16 bf16, two elements per 32-bit column) in TMEM
 __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(

@@ -382,7 +382,7 @@ int32_t try_split(holo_b200_ctx* ctx, const HoloCausalArgs& a, bool* taken) {
 //              buffer j % 2: tcgen05.ld half a row of S, cap, exponentiate, sum, tcgen05.st the bf16 weights
 // Without a running maximum O needs no correction: it stays in TMEM from the first tile to the last.
 // TMEM (all 512 columns): S at 0 and 128, O from 256; P at 384 and 448 where vdim leaves room, else over the S it came from,
-// each key half's weights over the first half of its scores (the next scores then wait for the item's product). It is allocated after the dependency wait, and dependents are
+// each key half's weights over the first half of its scores (the next scores then come behind the item's product). It is allocated after the dependency wait, and dependents are
 // released only after the allocation, so no neighbouring launch can hold columns this kernel or its predecessor waits for.
 constexpr int TILE_THREADS = 576;
 
@@ -487,7 +487,9 @@ causal_attention_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __
             // Item i is key tile i / NQ against query tile i % NQ, its scores in buffer i & 1. Between an item's weights and its
             // buffer's next scores lies what this one thread does, so it works on ready-made descriptors (a step of 16 k-elements
             // adds 32 bytes, four of them a chunk; a step of 16 keys adds 2048 bytes) and running stage numbers.
-            const uint64_t desc_q = smem_desc(s_q, 16, 1024), desc_k = smem_desc(s_k, 16, 1024), desc_v = smem_desc(s_v, TILE_CHUNK, 1024);
+            const uint64_t first_q = smem_desc(s_q, 16, 1024), first_v = smem_desc(s_v, TILE_CHUNK, 1024);
+            const uint32_t desc_q = (uint32_t)first_q, desc_k = (uint32_t)smem_desc(s_k, 16, 1024), high_s = (uint32_t)(first_q >> 32);
+            const uint32_t desc_v = (uint32_t)first_v, high_v = (uint32_t)(first_v >> 32);
             const uint32_t kstep = kbytes >> 4, vstep = vbytes >> 4;
             const bool alias = p.alias != 0;
             uint32_t ks = 0, kphase = 0, vs = 0, vphase = 0;
@@ -495,12 +497,19 @@ causal_attention_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __
                 const uint32_t qi = NQ == 2 ? i & 1u : 0u, buf = i & 1u;
                 if (qi == 0 && !mbar_wait(bar_k_full + 8 * ks, kphase, s_abort, p.status)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t dq = desc_q + qi * kstep, dk = desc_k + ks * kstep;
-                const uint32_t d = tmem_base + buf * 128;
-                for (uint32_t k0 = 0, off = 0; k0 < ksteps; k0 += 4, off += TILE_CHUNK >> 4) {
+                const uint32_t dq = desc_q + qi * kstep, dk = desc_k + ks * kstep, d = tmem_base + buf * 128;
+                if (ksteps == 8) {
 #pragma unroll
-                    for (uint32_t k = 0; k < 4; ++k)
-                        if (k0 + k < ksteps) umma_bf16(d, dq + off + 2 * k, dk + off + 2 * k, idesc_s, (k0 | k) != 0);
+                    for (uint32_t k = 0; k < 8; ++k) {
+                        const uint32_t off = (k >> 2) * (TILE_CHUNK >> 4) + 2 * (k & 3u);
+                        product_ss(d, dq + off, high_s, dk + off, high_s, idesc_s, k != 0);
+                    }
+                } else {
+                    for (uint32_t k0 = 0, off = 0; k0 < ksteps; k0 += 4, off += TILE_CHUNK >> 4) {
+#pragma unroll
+                        for (uint32_t k = 0; k < 4; ++k)
+                            if (k0 + k < ksteps) product_ss(d, dq + off + 2 * k, high_s, dk + off + 2 * k, high_s, idesc_s, (k0 | k) != 0);
+                    }
                 }
                 umma_commit(bar_s + 8 * buf);
                 if (qi == NQ - 1) {
@@ -519,15 +528,15 @@ causal_attention_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __
                 if (!alias && i + 2 < items) ok = scores(i + 2);
                 if (!ok) break;
                 const uint32_t tmem_p = tmem_base + (alias ? buf * 128 : 384 + buf * 64), d = tmem_o + qi * p.ostride, gap = alias ? 32 : 0;
-                const uint64_t dv = desc_v + vs * vstep;
+                const uint32_t dv = desc_v + vs * vstep;
 #pragma unroll
-                for (uint32_t k = 0; k < 8; ++k) umma_bf16_ts(d, tmem_p + k * 8 + (k >= 4 ? gap : 0), dv + 128 * k, idesc_o, k != 0 || i >= NQ);
+                for (uint32_t k = 0; k < 8; ++k) product_ts(d, tmem_p + k * 8 + (k >= 4 ? gap : 0), dv + 128 * k, high_v, idesc_o, k != 0 || i >= NQ);
                 umma_commit(bar_pv + 8 * buf);
                 if (qi == NQ - 1) {
                     umma_commit(bar_v_empty + 8 * vs);
                     if (++vs == p.vstages) vs = 0, vphase ^= 1;
                 }
-                if (alias && i + 2 < items) ok = mbar_wait(bar_pv + 8 * buf, phase, s_abort, p.status) && scores(i + 2);
+                if (alias && i + 2 < items) ok = scores(i + 2);      // behind the product that reads the weights there: one thread's products execute in order
             }
             if (ok) umma_commit(bar_o);
         }

@@ -544,7 +544,9 @@ window_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             // D = f32, A = B = bf16, M = 128; S: both operands K-major, N = 128; O: V is N-major, N = vdim
             const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
             const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((a.vdim >> 3) << 17) | ((128u >> 4) << 24);
-            const uint64_t desc_q = smem_desc(s_q, 16, 1024), desc_k = smem_desc(s_k, 16, 1024), desc_v = smem_desc(s_v, TILE_CHUNK, 1024);
+            const uint64_t first_q = smem_desc(s_q, 16, 1024), first_v = smem_desc(s_v, TILE_CHUNK, 1024);
+            const uint32_t desc_q = (uint32_t)first_q, desc_k = (uint32_t)smem_desc(s_k, 16, 1024), high_s = (uint32_t)(first_q >> 32);
+            const uint32_t desc_v = (uint32_t)first_v, high_v = (uint32_t)(first_v >> 32);
             uint32_t ks = 0, kphase = 0, vs = 0, vphase = 0;
             // S_q of the key tile whose chunks begin at slot ks; the last query tile gives every chunk back
             auto scores = [&](uint32_t q) {
@@ -553,10 +555,10 @@ window_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     if (q == 0 && !mbar_wait(bar_k_full + 8 * slot, phase, s_abort, p.status)) return false;
                     if (q == 0) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t width = c < p.chunks1 ? a.dim - 64 * c : a.dim2 - 64 * (c - p.chunks1);
-                    const uint64_t dq = desc_q + ((q * qbytes + c * TILE_CHUNK) >> 4), dk = desc_k + ((slot * TILE_CHUNK) >> 4);
+                    const uint32_t dq = desc_q + ((q * qbytes + c * TILE_CHUNK) >> 4), dk = desc_k + ((slot * TILE_CHUNK) >> 4);
 #pragma unroll
                     for (uint32_t k = 0; k < 4; ++k)
-                        if (16 * k < width) umma_bf16(tmem_base + q * 128, dq + 2 * k, dk + 2 * k, idesc_s, (c | k) != 0);
+                        if (16 * k < width) product_ss(tmem_base + q * 128, dq + 2 * k, high_s, dk + 2 * k, high_s, idesc_s, (c | k) != 0);
                     if (q == NQ - 1) umma_commit(bar_k_empty + 8 * slot);
                     if (++slot == p.kslots) slot = 0, phase ^= 1;
                 }
@@ -572,10 +574,10 @@ window_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     ok = ok && mbar_wait(bar_p + 8 * q, i & 1, s_abort, p.status);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t dv = desc_v + ((vs * vbytes) >> 4);
+                    const uint32_t dv = desc_v + ((vs * vbytes) >> 4);
 #pragma unroll
                     for (uint32_t k = 0; k < 8; ++k)
-                        umma_bf16_ts(tmem_base + 256 + q * 128, tmem_base + q * 128 + k * 8, dv + 128 * k, idesc_o, k != 0 || i != 0);
+                        product_ts(tmem_base + 256 + q * 128, tmem_base + q * 128 + k * 8, dv + 128 * k, high_v, idesc_o, k != 0 || i != 0);
                     umma_commit(bar_pv + 8 * q);
                     if (q == NQ - 1) {
                         umma_commit(bar_v_empty + 8 * vs);
