@@ -131,8 +131,15 @@ __device__ __forceinline__ float2 capped_exp_small(uint64_t s, uint64_t c0, uint
 // them. Warp w of split c takes 16-key tiles w, w + W, ... of the split's range through a private ring of STAGES tiles
 // (no block-wide synchronisation in the loop). Warps merge through shared memory, splits through a partial buffer: the
 // last CTA of a (kv head, row tile) to count in adds the partials in split order; nobody waits.
-// At short caches it is bound by latency, and instructions count: 16 heads over 4, dim 128, 1532 keys on the critical path of a
-// step 18 -> 12 us with copies that step through a tile by additions instead of divisions and four cells per thread in the merge.
+// At short caches it is bound by latency. Where one tile for each warp covers the cache (STAGES 1) there is no ring: 75 KiB of
+// shared memory in place of 209 let its CTAs start beside the ones of the product before it, which runs for 10 us more. They bring
+// their part of the cache into L2 meanwhile, and a warp's tile does not depend on the position. Every division that gives a place
+// stands before the wait, the queries are requested before the position is known, and in the last CTA a thread has twelve
+// splits' parts of its cells and of their row's sum on their way at a time and finishes them itself. 16 heads over 4, dim 128, on
+// the critical path of a step: 1532 keys 12 -> 7.5 us (of it 1.9 keys and values, 1.0 products and weights, 0.8 warps, 1.0
+// arrival, 0.9 parts, 0.6 result); alone 10.3 -> 7.5, 8192 rows of cache (three stages) 13.0 -> 10.8; four rows 15.9 -> 10.0; dim
+// 256 with eight rows 45.9 -> 19.0. Requesting by the position read before the wait, or going through the code once before it,
+// changed nothing.
 constexpr uint32_t SPLIT_SLOTS = 1024, SPLIT_SLOT_FLOATS = 16 * 257;
 
 struct SplitParams {
@@ -142,7 +149,7 @@ struct SplitParams {
     uint32_t group, splits;
 };
 
-template <int VT, int STAGES>   // vdim <= 16 VT
+template <int VT, int STAGES>   // vdim <= 16 VT; STAGES 1: the cache has one tile per warp at most
 __global__ void __launch_bounds__(256)
 causal_attention_split_kernel(const SplitParams p) {
     extern __shared__ __align__(16) uint8_t sm[];
@@ -154,22 +161,55 @@ causal_attention_split_kernel(const SplitParams p) {
     const uint32_t s_q = smem_u32(sm), s_ring = s_q + 16 * kp + warp * STAGES * tile_bytes;
     const uint32_t kv_ld = a.kv_heads * a.dim, vv_ld = a.kv_heads * a.vdim;
     holo_pdl_trigger();
-    holo_pdl_wait();
-    const uint32_t pos = *a.pos;
-    // the last position any row of this tile sees
-    const uint32_t last_row = min((z * 16 + 15) / p.group, a.rows - 1);
-    const uint32_t visible = min(pos + last_row + 1, a.cache_rows);
-    const uint32_t tiles = (visible + 15) / 16;
-    const uint32_t used = min(p.splits, (tiles + nwarps - 1) / nwarps);
-    if (split >= used) return;
-    const uint32_t t_begin = (uint32_t)((uint64_t)tiles * split / used), t_end = (uint32_t)((uint64_t)tiles * (split + 1) / used);
     const __nv_bfloat16* kbase = (const __nv_bfloat16*)a.k + g * a.dim;
     const __nv_bfloat16* vbase = (const __nv_bfloat16*)a.v + g * a.vdim;
     const uint32_t kvec = a.dim / 8, vvec = a.vdim / 8;
-
+    // the last position any row of this tile sees
+    const uint32_t last_row = min((z * 16 + 15) / p.group, a.rows - 1);
+    auto visible_at = [&](uint32_t at) { return (uint32_t)min((uint64_t)at + last_row + 1, (uint64_t)a.cache_rows); };
+    // The position before the wait is a guess: the kernel ahead, or one ahead of it, may still write it. It only chooses which
+    // rows of the cache to bring into L2 meanwhile, and is read past L1 so that the read after the wait cannot meet it there.
+    auto read_pos = [&] {
+        uint32_t v;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.pos) : "memory");
+        return v;
+    };
+    if (STAGES == 1) {
+        const uint32_t guess = visible_at(read_pos()), from = split * nwarps * 16, to = min(guess, from + nwarps * 16);
+        const uint32_t klines = (a.dim * 2 + 127) / 128, vlines = (a.vdim * 2 + 127) / 128;
+        for (uint32_t key = from + threadIdx.x; key < to; key += blockDim.x) {
+            for (uint32_t i = 0; i < klines; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(kbase + (uint64_t)key * kv_ld + 64 * i));
+            for (uint32_t i = 0; i < vlines; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(vbase + (uint64_t)key * vv_ld + 64 * i));
+        }
+    }
     // A warp copies a tile 32 vectors at a time; the place moves on by additions (a division per vector cost more than the copy)
     const uint32_t krow = lane / kvec, kcol = lane % kvec, krows = 32 / kvec, kcols = 32 % kvec;
     const uint32_t vrow = lane / vvec, vcol = lane % vvec, vrows = 32 / vvec, vcols = 32 % vvec;
+    auto request_q = [&](uint32_t r, uint32_t c, uint32_t row, uint32_t of) {     // rows past the step's last one are zero
+        const uint64_t at = ((uint64_t)min(row, a.rows - 1) * a.heads + g * p.group + of) * a.dim + c * 8;
+        cp_async16(s_q + r * kp + c * 16, (const __nv_bfloat16*)a.q + at, row < a.rows);
+    };
+    const uint32_t qr0 = threadIdx.x / kvec, qc0 = threadIdx.x % kvec, qrow0 = (z * 16 + qr0) / p.group, qof0 = (z * 16 + qr0) % p.group;
+    const uint32_t r0 = lane >> 2;                        // this thread's rows of the tile: r0 and r0 + 8
+    const uint32_t row_of[2] = {min((z * 16 + r0) / p.group, a.rows - 1), min((z * 16 + r0 + 8) / p.group, a.rows - 1)};
+    const uint32_t nrows = min(16u, a.rows * p.group - z * 16), vquads = a.vdim / 4, cells = nrows * vquads;
+    const uint32_t cell_row0 = threadIdx.x / vquads, cell_col0 = threadIdx.x % vquads;
+    holo_pdl_wait();
+    // the queries' place does not depend on the position
+    if (qr0 < 16) request_q(qr0, qc0, qrow0, qof0);
+    const uint32_t pos = STAGES == 1 ? read_pos() : *a.pos;
+    const float sink0 = a.sink && cell_row0 < nrows ? a.sink[g * p.group + (z * 16 + cell_row0) % p.group] : 0.0f;
+    for (uint32_t i = threadIdx.x + blockDim.x; i < 16 * kvec; i += blockDim.x) request_q(i / kvec, i % kvec, (z * 16 + i / kvec) / p.group, (z * 16 + i / kvec) % p.group);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const uint32_t visible = visible_at(pos);
+    const uint32_t tiles = (visible + 15) / 16;
+    const uint32_t used = min(p.splits, (tiles + nwarps - 1) / nwarps);
+    if (split >= used) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        return;
+    }
+    const uint32_t t_begin = STAGES == 1 ? split * nwarps : (uint32_t)((uint64_t)tiles * split / used);
+    const uint32_t t_end = STAGES == 1 ? min(tiles, t_begin + nwarps) : (uint32_t)((uint64_t)tiles * (split + 1) / used);
     auto load_rows = [&](uint32_t dst, uint32_t pitch, const __nv_bfloat16* src, uint32_t ld, uint32_t first, uint32_t vecs, uint32_t r, uint32_t c, uint32_t dr, uint32_t dc) {
 #pragma unroll 4
         while (r < 16) {
@@ -187,32 +227,24 @@ causal_attention_split_kernel(const SplitParams p) {
     };
     const uint32_t first = t_begin + warp;
 #pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) {
+    for (int s = 0; s < (STAGES == 1 ? 1 : STAGES - 1); ++s) {
         const uint32_t t = first + s * nwarps;
         if (t < t_end) load_tile(t, s);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    // the query tile (rows past the step's last one are zero)
-    for (uint32_t i = threadIdx.x; i < 16 * kvec; i += blockDim.x) {
-        const uint32_t r = i / kvec, c = i % kvec, qr = z * 16 + r, row = qr / p.group;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (row < a.rows) v = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)a.q + ((uint64_t)row * a.heads + g * p.group + qr % p.group) * a.dim + c * 8);
-        *reinterpret_cast<uint4*>(sm + r * kp + c * 16) = v;
-    }
-    __syncthreads();
-
-    const uint32_t r0 = lane >> 2;                        // this thread's rows of the tile: r0 and r0 + 8
     const float c2 = a.softcap * LOG2E;
     float c1[2];
     uint32_t limit[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-        const uint32_t row = min((z * 16 + r0 + 8 * e) / p.group, a.rows - 1);
-        c1[e] = 2.0f * LOG2E * a.scale * query_factor(pos + row, a.temp_coef, a.temp_every) / a.softcap;
-        limit[e] = pos + row;
+        c1[e] = 2.0f * LOG2E * a.scale * query_factor(pos + row_of[e], a.temp_coef, a.temp_every) / a.softcap;
+        limit[e] = pos + row_of[e];
     }
     // with at most eight rows the upper half of the tile is all padding
     const bool upper = a.rows * p.group > z * 16 + 8;
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES == 1 ? 0 : STAGES - 1) : "memory");
+    __syncthreads();     // the queries of all threads
+
     float o[VT][2][4];
     float sum[2] = {0.0f, 0.0f};
 #pragma unroll
@@ -225,9 +257,9 @@ causal_attention_split_kernel(const SplitParams p) {
     const uint32_t ksteps = a.dim / 16, vsteps = a.vdim / 16;
     uint32_t stage = 0;
     for (uint32_t t = first; t < t_end; t += nwarps) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES == 1 ? 0 : STAGES - 2) : "memory");
         __syncwarp();
-        {   // refill the stage the previous iteration has emptied
+        if (STAGES > 1) {   // refill the stage the previous iteration has emptied
             const uint32_t nt = t + (STAGES - 1) * nwarps;
             if (nt < t_end) load_tile(nt, stage == 0 ? STAGES - 1 : stage - 1);
             asm volatile("cp.async.commit_group;" ::: "memory");
@@ -272,61 +304,83 @@ causal_attention_split_kernel(const SplitParams p) {
         sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], 1);
         sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], 2);
     }
-    __syncthreads();   // every warp is through with its ring: it becomes the merge buffer [warp][16][vdim + 1]
+    __syncthreads();   // every warp is through with its ring: it becomes the merge buffer [warp][16][vdim + 8], a row's sum behind its cells
     float* merge = reinterpret_cast<float*>(sm);
-    const uint32_t ml = a.vdim + 1;
+    const uint32_t ml = a.vdim + 8;      // rows eight banks apart
     float* mine = merge + (size_t)warp * 16 * ml;
 #pragma unroll
-    for (int n = 0; n < VT; ++n)
-        if ((uint32_t)n < vsteps)
+    for (int h = 0; h < 2; ++h)
+        if (r0 + 8 * h < nrows) {
+            float* row = mine + (r0 + 8 * h) * ml;
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+            for (int n = 0; n < VT; ++n)
+                if ((uint32_t)n < vsteps)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) mine[(r0 + 8 * (e >> 1)) * ml + n * 16 + h * 8 + (lane & 3) * 2 + (e & 1)] = o[n][h][e];
-    if ((lane & 3) == 0) {
-        mine[r0 * ml + a.vdim] = sum[0];
-        mine[(r0 + 8) * ml + a.vdim] = sum[1];
-    }
+                    for (int x = 0; x < 2; ++x) *reinterpret_cast<float2*>(row + n * 16 + x * 8 + (lane & 3) * 2) = make_float2(o[n][x][2 * h], o[n][x][2 * h + 1]);
+            if ((lane & 3) == 0) row[a.vdim] = sum[h];
+        }
     __syncthreads();
-    const uint32_t nrows = min(16u, a.rows * p.group - z * 16), cells = nrows * ml;
     const uint32_t tile_id = z * a.kv_heads + g;
-    float* part = p.partials + ((uint64_t)tile_id * p.splits + split) * SPLIT_SLOT_FLOATS;
-    for (uint32_t i = threadIdx.x; i < cells; i += blockDim.x) {
-        float v = 0.0f;
-        for (uint32_t w = 0; w < nwarps; ++w) v += merge[(size_t)w * 16 * ml + i];
-        if (used == 1) merge[i] = v;     // only this thread touches cell i of every warp's part
-        else __stcg(part + i, v);
-    }
-    if (used > 1) {
-        __shared__ uint32_t s_last;
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) s_last = atomicAdd(p.arrivals + tile_id, 1u) == used - 1 ? 1u : 0u;
-        __syncthreads();
-        if (!s_last) return;
-        __threadfence();
-        if (threadIdx.x == 0) p.arrivals[tile_id] = 0;
-        const float* all = p.partials + (uint64_t)tile_id * p.splits * SPLIT_SLOT_FLOATS;
-        // four cells of a thread at a time, so that more than one cell's parts are on their way
-        for (uint32_t i = threadIdx.x; i < cells; i += 4 * blockDim.x) {
-            float v[4] = {};
+    float* part = p.partials + ((uint64_t)tile_id * p.splits + split) * SPLIT_SLOT_FLOATS;    // cells, then the rows' sums
+    auto finish = [&](uint32_t r, uint32_t c, float total, const float4& v) {
+        const uint32_t qr = z * 16 + r, head = g * p.group + qr % p.group;
+        const float sink = r == cell_row0 ? sink0 : a.sink ? a.sink[head] : 0.0f;
+        const float inv = __fdiv_rn(1.0f, total + (a.sink ? ex2(sink * LOG2E) : 0.0f));
+        __nv_bfloat16* to = (__nv_bfloat16*)a.out + (uint64_t)(qr / p.group) * a.ld + head * a.vdim + 4 * c;
+        *reinterpret_cast<uint32_t*>(to) = pack_bf16(v.x * inv, v.y * inv);
+        *reinterpret_cast<uint32_t*>(to + 2) = pack_bf16(v.z * inv, v.w * inv);
+    };
+    auto add = [](float4& v, const float4& w) { v.x += w.x, v.y += w.y, v.z += w.z, v.w += w.w; };
+    // four cells of a row for each thread, which adds up the row's sum as well
+    for (uint32_t i = threadIdx.x, r = cell_row0, c = cell_col0; i < cells; i += blockDim.x, r = i / vquads, c = i % vquads) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        float total = 0.0f;
 #pragma unroll 8
-            for (uint32_t c = 0; c < used; ++c)
-#pragma unroll
-                for (uint32_t x = 0; x < 4; ++x)
-                    if (i + x * blockDim.x < cells) v[x] += __ldcg(all + (uint64_t)c * SPLIT_SLOT_FLOATS + i + x * blockDim.x);
-#pragma unroll
-            for (uint32_t x = 0; x < 4; ++x)
-                if (i + x * blockDim.x < cells) merge[i + x * blockDim.x] = v[x];
+        for (uint32_t w = 0; w < nwarps; ++w) {
+            const float* row = merge + ((size_t)w * 16 + r) * ml;
+            add(v, *reinterpret_cast<const float4*>(row + 4 * c));
+            total += row[a.vdim];
+        }
+        if (used == 1) {
+            finish(r, c, total, v);
+        } else {
+            __stcg(reinterpret_cast<float4*>(part) + i, v);
+            if (c == 0) __stcg(part + 16 * a.vdim + r, total);
         }
     }
+    if (used == 1) return;
+    __shared__ uint32_t s_last;
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < nrows * (a.vdim / 2); i += blockDim.x) {
-        const uint32_t r = i / (a.vdim / 2), c = 2 * (i % (a.vdim / 2)), qr = z * 16 + r, head = g * p.group + qr % p.group;
-        const float denom = merge[r * ml + a.vdim] + (a.sink ? ex2(a.sink[head] * LOG2E) : 0.0f);
-        const float inv = __fdiv_rn(1.0f, denom);
-        *reinterpret_cast<uint32_t*>((__nv_bfloat16*)a.out + (uint64_t)(qr / p.group) * a.ld + head * a.vdim + c) =
-            pack_bf16(merge[r * ml + c] * inv, merge[r * ml + c + 1] * inv);
+    if (threadIdx.x == 0) {     // the barrier orders the others' stores before this fence
+        __threadfence();
+        s_last = atomicAdd(p.arrivals + tile_id, 1u) == used - 1 ? 1u : 0u;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
+    if (threadIdx.x == 0) p.arrivals[tile_id] = 0;
+    const float* all = p.partials + (uint64_t)tile_id * p.splits * SPLIT_SLOT_FLOATS;
+    for (uint32_t i = threadIdx.x, r = cell_row0, c = cell_col0; i < cells; i += blockDim.x, r = i / vquads, c = i % vquads) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        float total = 0.0f;
+        // the parts and sums of MERGE splits are on their way at a time, those of the last, ragged group too
+        constexpr uint32_t MERGE = 12;
+        for (uint32_t c0 = 0; c0 < used; c0 += MERGE) {
+            float4 one[MERGE];
+            float sums[MERGE];
+#pragma unroll
+            for (uint32_t x = 0; x < MERGE; ++x) {
+                const float* at = all + (uint64_t)(c0 + x) * SPLIT_SLOT_FLOATS;
+                one[x] = c0 + x < used ? __ldcg(reinterpret_cast<const float4*>(at) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                sums[x] = c0 + x < used ? __ldcg(at + 16 * a.vdim + r) : 0.0f;
+            }
+#pragma unroll
+            for (uint32_t x = 0; x < MERGE; ++x) {
+                add(v, one[x]);
+                total += sums[x];
+            }
+        }
+        finish(r, c, total, v);
     }
 }
 
@@ -348,10 +402,13 @@ int32_t try_split(holo_b200_ctx* ctx, const HoloCausalArgs& a, bool* taken) {
     const uint32_t group = a.heads / a.kv_heads, qtiles = (a.rows * group + 15) / 16;
     const uint32_t pairs = qtiles * a.kv_heads;
     if (a.vdim > 256 || a.dim > 256 || pairs > SPLIT_SLOTS || qtiles > 65535) return HOLO_OK;
-    const int stages = a.vdim <= 64 ? 4 : a.vdim <= 128 ? 3 : 2;
+    int stages = a.vdim <= 64 ? 4 : a.vdim <= 128 ? 3 : 2;
     const size_t kp = a.dim * 2 + 16, vp = a.vdim * 2 + 16, limit = (size_t)ctx->smem_optin - 1024;
     uint32_t warps = 8;
-    auto bytes = [&](uint32_t w) { return std::max(16 * kp + w * stages * 16 * (kp + vp), (size_t)w * 16 * (a.vdim + 1) * 4); };
+    // a tile per warp is all that there is: no ring, and the kernels before and after fit on the same SMs
+    const uint32_t splits = std::max(1u, (uint32_t)ctx->sm_count / pairs);
+    if ((uint64_t)splits * warps * 16 >= a.cache_rows) stages = 1;
+    auto bytes = [&](uint32_t w) { return std::max(16 * kp + w * stages * 16 * (kp + vp), (size_t)w * 16 * (a.vdim + 8) * 4); };
     while (warps > 1 && bytes(warps) > limit) warps /= 2;
     if (bytes(warps) > limit) return HOLO_OK;
     if (!ctx->causal_partials) HOLO_CUDA(cudaMalloc(&ctx->causal_partials, (size_t)SPLIT_SLOTS * SPLIT_SLOT_FLOATS * 4));
@@ -360,11 +417,13 @@ int32_t try_split(holo_b200_ctx* ctx, const HoloCausalArgs& a, bool* taken) {
     p.partials = ctx->causal_partials;
     p.arrivals = ctx->attn_arrivals;
     p.group = group;
-    p.splits = (uint32_t)ctx->sm_count / pairs;
-    const uint32_t most = (a.cache_rows + 16 * warps - 1) / (16 * warps);
-    if (p.splits > most) p.splits = most;
-    if (p.splits < 1) p.splits = 1;
+    p.splits = std::max(1u, std::min(splits, (a.cache_rows + 16 * warps - 1) / (16 * warps)));
     *taken = true;
+    if (stages == 1) {
+        if (a.vdim <= 64) return launch_split<4, 1>(ctx, p, qtiles, warps, bytes(warps));
+        if (a.vdim <= 128) return launch_split<8, 1>(ctx, p, qtiles, warps, bytes(warps));
+        return launch_split<16, 1>(ctx, p, qtiles, warps, bytes(warps));
+    }
     if (a.vdim <= 64) return launch_split<4, 4>(ctx, p, qtiles, warps, bytes(warps));
     if (a.vdim <= 128) return launch_split<8, 3>(ctx, p, qtiles, warps, bytes(warps));
     return launch_split<16, 2>(ctx, p, qtiles, warps, bytes(warps));

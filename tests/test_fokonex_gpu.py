@@ -6,6 +6,7 @@ import sys
 
 import numpy as np
 import pytest
+import torch
 
 import fokonex_reference as ref
 from hologram_b200 import kernel_call as kc
@@ -285,6 +286,21 @@ def test_attention_splits_give_the_same_bits_as_repeats(backend):
     first = run_attention(backend, q, k, v, 2998, 0.125, 20.0, 0.2, 64, sinks, BF)
     for _ in range(3):
         assert np.array_equal(run_attention(backend, q, k, v, 2998, 0.125, 20.0, 0.2, 64, sinks, BF), first)
+
+
+@pytest.mark.parametrize("extra", [0, 1], ids=["one-tile-a-warp", "ring"])
+@pytest.mark.parametrize("shape", [(1, 8, 8, 32, 32), (3, 12, 4, 48, 80), (2, 8, 2, 80, 128), (5, 8, 2, 64, 176), (17, 2, 1, 256, 256)], ids=lambda s: "-".join(map(str, s)))
+def test_attention_of_few_rows_around_the_longest_cache_without_a_ring(backend, shape, extra):
+    """A cache that one 16-key tile for each of the chip's warps covers takes no ring; one row more does. Positions at the edges of tiles, CTAs and the cache."""
+    rows, heads, groups, dim, vdim = shape
+    splits = torch.cuda.get_device_properties(0).multi_processor_count // (-(-rows * heads // groups // 16) * groups)
+    cache = splits * 8 * 16 + extra
+    q, k, v, sinks = random_attention(rows, heads, groups, dim, vdim, cache, seed=rows + dim)
+    for first in (0, 15, 128 - rows, 129 - rows, 130 - rows, cache // 2, cache - rows):
+        seen = first + rows
+        got = run_attention(backend, q, k[:seen], v[:seen], first, dim ** -0.5, 25.0, 0.3, 16, sinks, BF, cache, stale=np.inf)
+        want = ref.attention(q, k[:seen], v[:seen], first, dim ** -0.5, 25.0, 0.3, 16, sinks)
+        assert np.abs(got - want).max() / np.abs(want).max() < 1e-2, first      # weights and results in bf16, as above
 
 
 # ---- whole models ----
