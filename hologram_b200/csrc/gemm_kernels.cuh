@@ -194,9 +194,9 @@ __device__ __forceinline__ void lin_rotate(const GemmParams& p, const GemmLin& g
             v[2 * i + 1] = b * t[i].x + a * t[i].y;
         }
 }
-// Store N consecutive finished cells of one row, of which `left` exist.
+// Store N consecutive finished cells of one row, of which `left` exist. Not `live`: everything but the stores.
 template <int N>
-__device__ __forceinline__ void lin_put(const GemmLin& g, uint64_t idx, uint32_t left, float (&v)[N]) {
+__device__ __forceinline__ void lin_put(const GemmLin& g, uint64_t idx, uint32_t left, float (&v)[N], bool live = true) {
     const bool full = N <= left;
     if (g.f32) {
         float* out = reinterpret_cast<float*>(g.out) + idx;
@@ -210,11 +210,15 @@ __device__ __forceinline__ void lin_put(const GemmLin& g, uint64_t idx, uint32_t
                 }
             }
 #pragma unroll
-            for (int i = 0; i + 3 < N; i += 4) *reinterpret_cast<float4*>(out + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            for (int i = 0; i + 3 < N; i += 4)
+                if (live) *reinterpret_cast<float4*>(out + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
         } else {
 #pragma unroll
             for (int i = 0; i < N; ++i)
-                if ((uint32_t)i < left) out[i] = v[i] + (res ? res[i] : 0.0f);
+                if ((uint32_t)i < left) {
+                    const float r = res ? res[i] : 0.0f;
+                    if (live) out[i] = v[i] + r;
+                }
         }
     } else {
         __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(g.out) + idx;
@@ -227,24 +231,24 @@ __device__ __forceinline__ void lin_put(const GemmLin& g, uint64_t idx, uint32_t
                     const __nv_bfloat162 h = __floats2bfloat162_rn(v[i + 2 * x], v[i + 2 * x + 1]);
                     w[x] = *reinterpret_cast<const uint32_t*>(&h);
                 }
-                *reinterpret_cast<uint4*>(out + i) = make_uint4(w[0], w[1], w[2], w[3]);
+                if (live) *reinterpret_cast<uint4*>(out + i) = make_uint4(w[0], w[1], w[2], w[3]);
             }
         } else if (N % 4 == 0 && full && ((uintptr_t)out & 7u) == 0) {
 #pragma unroll
             for (int i = 0; i + 3 < N; i += 4) {
                 const __nv_bfloat162 lo = __floats2bfloat162_rn(v[i], v[i + 1]), hi = __floats2bfloat162_rn(v[i + 2], v[i + 3]);
-                *reinterpret_cast<uint2*>(out + i) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                if (live) *reinterpret_cast<uint2*>(out + i) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
             }
         } else {
 #pragma unroll
             for (int i = 0; i < N; ++i)
-                if ((uint32_t)i < left) out[i] = __float2bfloat16_rn(v[i]);
+                if (live && (uint32_t)i < left) out[i] = __float2bfloat16_rn(v[i]);
         }
     }
 }
 // Finish and store N consecutive cells of one row (N a multiple of 4, the cells in one segment).
 template <int N>
-__device__ __forceinline__ void lin_store(const GemmParams& p, uint32_t row, uint32_t col, const float (&acc)[N]) {
+__device__ __forceinline__ void lin_store(const GemmParams& p, uint32_t row, uint32_t col, const float (&acc)[N], bool live = true) {
     const GemmLin& g = p.lin[lin_segment(p, col)];
     const uint32_t c = col - g.col_begin, width = g.width;
     if (c >= width) return;
@@ -256,7 +260,7 @@ __device__ __forceinline__ void lin_store(const GemmParams& p, uint32_t row, uin
         float v[N / 2];
 #pragma unroll
         for (int i = 0; i < N / 2; ++i) v[i] = alpha * (sigmoid_times<true>(acc[2 * i], acc[2 * i]) * acc[2 * i + 1]);
-        lin_put<N / 2>(g, orow * g.ld + (c >> 1), (width - c) >> 1, v);
+        lin_put<N / 2>(g, orow * g.ld + (c >> 1), (width - c) >> 1, v, live);
         return;
     }
     float v[N];
@@ -277,7 +281,7 @@ __device__ __forceinline__ void lin_store(const GemmParams& p, uint32_t row, uin
     if (g.rot_head) lin_rotate<N>(p, g, row, c, v);
 #pragma unroll
     for (int i = 0; i < N; ++i) v[i] *= alpha;
-    lin_put<N>(g, orow * g.ld + c, width - c, v);
+    lin_put<N>(g, orow * g.ld + c, width - c, v, live);
 }
 // 32 accumulator columns of one row straight from TMEM registers.
 __device__ __forceinline__ void lin_store32(const GemmParams& p, uint32_t row, uint32_t col0, const uint32_t (&v)[32]) {
@@ -415,6 +419,14 @@ struct GemmSmem {
     static constexpr uint32_t RING = STAGES * STAGE + (BM - A_ROWS) * BK * 2;  // tail pad: the last A read stays in bounds
     static constexpr uint32_t BARS = (RING + 1023u) & ~1023u;   // full[STAGES], empty[STAGES], accum, tmem slot, abort, flag
     static constexpr uint32_t TOTAL = BARS + 256 + 1024;
+    // Few rows: the partial sums of a K split are written into the shared memory of the CTA that adds them up, into the tail pad
+    // behind the ring (what the MMA makes of those bytes is never stored): [split][row][BN] of at most 21 rows (7 splits). That
+    // saves the round trip of reading them there and the second cluster barrier. After the last MMA of a one-row Linear product of
+    // 2048 x 1344 in eight splits 3.5 us passed until its end; so, and with the rows' way out gone through beforehand (add_up in
+    // the kernel), 2.1. A token of a five-run decoder 357 -> 337 us, of a four-layer one 152 -> 145.
+    static constexpr bool PUSH = A_ROWS == 16 && BN <= 128;
+    static constexpr uint32_t PUSHED = STAGES * STAGE;
+    static_assert(!PUSH || 21 * BN * 4 <= (BM - A_ROWS) * BK * 2, "the parts fit in the tail pad");
 };
 
 // AR: the instantiation whose epilogue carries the tensor-parallel sum; the plain one compiles none of it
@@ -456,6 +468,8 @@ matmul_bf16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // whoever writes into another CTA's shared memory waits for this first: that CTA has begun
+    if (S::PUSH && p.splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     const uint32_t tmem_base = *s_tmem;
     // A constant B (a weight nothing in the stream rewrites) does not depend on the previous kernel: the first
     // ring-full of its tiles is requested before the wait, so those bytes are on their way (or already here)
@@ -472,6 +486,7 @@ matmul_bf16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                 tma_load_2d(st + S::A_BYTES + h * (BK * 128), &map_b, (int)(n0 + 64 * h), k0, bar_full + 8 * i);
         }
     }
+    const int a_k0 = LIN ? (int)p.lin[lin_segment(p, n0)].k_offset : 0;
     holo_pdl_wait();  // barriers and TMEM were set up while the previous kernel drained
     uint32_t m_end = p.m, a_row = m0, b_row = 0;
     if (LIN) {
@@ -486,7 +501,6 @@ matmul_bf16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         // ---------------- TMA producer ----------------
         if (lane == 0) {
             const uint32_t tx = p.box_m * BK * 2 + S::B_BYTES;
-            const int a_k0 = LIN ? (int)p.lin[lin_segment(p, n0)].k_offset : 0;
             // after an abort nothing new is requested, but the stages whose B tiles are already in flight still get
             // their A tiles: their barriers then complete and the loop below sees the copies land before the CTA ends
             const uint32_t todo = *s_abort ? pre : nkb;
@@ -538,142 +552,205 @@ matmul_bf16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         const uint32_t row = m0 + quarter * 32 + lane;
         // an earlier launch gave up on a wait: store nothing (the round trip to the status word overlaps the mainloop)
         if (warp == 2 && lane == 0 && (*reinterpret_cast<volatile uint32_t*>(p.status) & 4u)) *s_abort = 1;
-        if (nkb != 0) mbar_wait(bar_accum, 0, s_abort, p.status);
-        asm volatile("bar.sync 1, 128;" ::: "memory");   // all four epilogue warps see the same abort state
-        const bool ok = !*s_abort;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (LIN && ok && p.splits == 1) {
-#pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
-                uint32_t v[32];
-                tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (uint32_t)(c * 32), v);
-                const uint32_t col0 = n0 + c * 32;
-                if (row < m_end && col0 < p.n) lin_store32(p, row, col0, v);
-            }
-        } else if (!LIN && ok && p.splits == 1 && p.gated) {
-            if constexpr (BN == 128) {
-                const uint32_t half_n = p.n >> 1;
-#pragma unroll 1
-                for (int c = 0; c < 2; ++c) {
-                    uint32_t v[32], w[32];
-                    tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (uint32_t)(c * 32), v);
-                    tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (uint32_t)(64 + c * 32), w);
-                    const uint32_t col0 = (n0 >> 1) + c * 32;
-                    if (row < p.m && col0 < half_n) {
-                        uint16_t* dst = p.seg[0].out + (uint64_t)row * half_n + col0;
-                        uint32_t packed[16];
+        const bool pushes = S::PUSH && p.splits > 1;
+        // A Linear product's rows that this CTA adds up: first without sums and without storing, while the products are still
+        // running, so that the code, the parameters, the residual, the place and the rotation are in the caches when the sums
+        // arrive (1.5 us of the 2048 x 1344 product; gone through before the dependency wait as well it saved nothing more)
+        const uint32_t parts = base + S::PUSHED, part_pitch = ((15u + p.splits) / p.splits) * (BN * 4);
+        auto add_up = [&](bool live) {
+            for (uint32_t rl = split + p.splits * (warp - 2), at = (warp - 2) * (BN * 4); rl < m_end - m0; rl += 4 * p.splits, at += 4 * BN * 4) {
+                if (lane >= BN / 4 || n0 + 4 * lane >= p.n) continue;
+                float4 part[8];
 #pragma unroll
-                        for (int x = 0; x < 16; ++x) {
-                            const uint16_t lo = gated_elem<F16>(__uint_as_float(v[2 * x]), __uint_as_float(w[2 * x]), p.seg[0].table);
-                            const uint16_t hi = gated_elem<F16>(__uint_as_float(v[2 * x + 1]), __uint_as_float(w[2 * x + 1]), p.seg[0].table);
-                            packed[x] = (uint32_t)lo | ((uint32_t)hi << 16);
-                        }
-#pragma unroll
-                        for (int x = 0; x < 4; ++x)
-                            reinterpret_cast<uint4*>(dst)[x] = make_uint4(packed[4 * x], packed[4 * x + 1], packed[4 * x + 2], packed[4 * x + 3]);
-                    }
+                for (uint32_t sidx = 0; sidx < 8; ++sidx) {
+                    part[sidx] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (sidx < p.splits)
+                        asm volatile("ld.shared::cta.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(part[sidx].x), "=f"(part[sidx].y), "=f"(part[sidx].z), "=f"(part[sidx].w)
+                                     : "r"(parts + sidx * part_pitch + at + lane * 16) : "memory");
                 }
-            }
-        } else if (!LIN && ok && p.splits == 1 && (AR && p.ar_world > 1)) {
-            // tensor-parallel sum in the epilogue: first push every unit of this thread's row, then
-            // collect the peers' units (the NVLink latency of all pushes overlaps)
-            const GemmSeg sg = p.seg[0];
-#pragma unroll 1
-            for (int pass = 0; pass < 2; ++pass) {
-#pragma unroll 1
-                for (int c = 0; c < BN / 32; ++c) {
-                    uint32_t v[32];
-                    tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (uint32_t)(c * 32), v);
-                    const uint32_t col0 = n0 + c * 32;
-                    if (row >= p.m || col0 >= p.n) continue;
-#pragma unroll 1
-                    for (int x = 0; x < 8; ++x) {
-                        if (col0 + 4 * x >= p.n) break;
-                        const float mine4[4] = {__uint_as_float(v[4 * x]), __uint_as_float(v[4 * x + 1]), __uint_as_float(v[4 * x + 2]),
-                                                __uint_as_float(v[4 * x + 3])};
-                        const uint2 mine = ar_pack<F16>(mine4);
-                        const uint64_t idx = (uint64_t)row * p.n + col0 + 4 * x, unit = idx >> 2;
-                        if (pass == 0) {
-                            ar_push(p, ar_epoch, ar_units, unit, mine);
-                            continue;
-                        }
-                        float a4[4];
-                        if (!ar_sum<F16>(p, ar_epoch, ar_units, unit, mine, a4)) {
-                            atomicOr(p.status, 8u);
-                            continue;
-                        }
-                        uint16_t h[4];
+                float4 acc = part[0];
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) h[e] = epilogue_elem<F16>(a4[e], nullptr, sg.residual, idx + e);
-                        *reinterpret_cast<uint2*>(sg.out + idx) = make_uint2((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16));
+                for (uint32_t sidx = 1; sidx < 8; ++sidx)
+                    if (sidx < p.splits) { acc.x += part[sidx].x; acc.y += part[sidx].y; acc.z += part[sidx].z; acc.w += part[sidx].w; }
+                const float a4[4] = {acc.x, acc.y, acc.z, acc.w};
+                lin_store<4>(p, m0 + rl, n0 + 4 * lane, a4, live);
+            }
+        };
+        bool ok = true;
+#pragma unroll 1
+        for (uint32_t live = LIN && pushes ? 0 : 1; live < 2; ++live) {
+            if (live) {
+                if (nkb != 0) mbar_wait(bar_accum, 0, s_abort, p.status);
+                asm volatile("bar.sync 1, 128;" ::: "memory");   // all four epilogue warps see the same abort state
+                ok = !*s_abort;
+                if (pushes) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (LIN && ok && p.splits == 1) {
+#pragma unroll 1
+                    for (int c = 0; c < BN / 32; ++c) {
+                        uint32_t v[32];
+                        tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (uint32_t)(c * 32), v);
+                        const uint32_t col0 = n0 + c * 32;
+                        if (row < m_end && col0 < p.n) lin_store32(p, row, col0, v);
                     }
-                }
-            }
-        } else if (!LIN && ok && p.splits == 1) {
+                } else if (!LIN && ok && p.splits == 1 && p.gated) {
+                    if constexpr (BN == 128) {
+                        const uint32_t half_n = p.n >> 1;
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
-                uint32_t v[32];
-                tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (uint32_t)(c * 32), v);
-                const uint32_t col0 = n0 + c * 32;
-                if (row < p.m && col0 < p.n) {
-                    uint32_t si = 0;
-                    while (si + 1 < p.nseg && col0 >= p.seg[si].col_end) ++si;
-                    const GemmSeg sg = p.seg[si];
-                    const uint64_t idx0 = (uint64_t)row * (sg.col_end - sg.col_begin) + (col0 - sg.col_begin);
-                    uint16_t* dst = sg.out + idx0;
-                    if (col0 + 32 <= sg.col_end && ((uintptr_t)dst & 15u) == 0) {
-                        uint32_t w[16];
+                        for (int c = 0; c < 2; ++c) {
+                            uint32_t v[32], w[32];
+                            tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (uint32_t)(c * 32), v);
+                            tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (uint32_t)(64 + c * 32), w);
+                            const uint32_t col0 = (n0 >> 1) + c * 32;
+                            if (row < p.m && col0 < half_n) {
+                                uint16_t* dst = p.seg[0].out + (uint64_t)row * half_n + col0;
+                                uint32_t packed[16];
 #pragma unroll
-                        for (int x = 0; x < 16; ++x) {
-                            uint16_t lo = epilogue_elem<F16>(__uint_as_float(v[2 * x]), sg.table, sg.residual, idx0 + 2 * x);
-                            uint16_t hi = epilogue_elem<F16>(__uint_as_float(v[2 * x + 1]), sg.table, sg.residual, idx0 + 2 * x + 1);
-                            w[x] = (uint32_t)lo | ((uint32_t)hi << 16);
-                        }
+                                for (int x = 0; x < 16; ++x) {
+                                    const uint16_t lo = gated_elem<F16>(__uint_as_float(v[2 * x]), __uint_as_float(w[2 * x]), p.seg[0].table);
+                                    const uint16_t hi = gated_elem<F16>(__uint_as_float(v[2 * x + 1]), __uint_as_float(w[2 * x + 1]), p.seg[0].table);
+                                    packed[x] = (uint32_t)lo | ((uint32_t)hi << 16);
+                                }
 #pragma unroll
-                        for (int x = 0; x < 4; ++x)
-                            reinterpret_cast<uint4*>(dst)[x] = make_uint4(w[4 * x], w[4 * x + 1], w[4 * x + 2], w[4 * x + 3]);
-                    } else {
-#pragma unroll
-                        for (int x = 0; x < 32; ++x)
-                            if (col0 + x < sg.col_end) dst[x] = epilogue_elem<F16>(__uint_as_float(v[x]), sg.table, sg.residual, idx0 + x);
-                    }
-                }
-            }
-        } else if (ok) {
-            // split-K: park this CTA's f32 accumulator rows in the (now idle) ring; 16-byte units of a
-            // row are XOR-swizzled with the row number so that the 32 rows of a warp do not hit one bank
-            const uint32_t row_local = quarter * 32 + lane;
-            if (m0 + quarter * 32 < m_end) {  // warp-uniform: the TMEM load is a whole-warp instruction
-#pragma unroll 1
-                for (int c = 0; c < BN / 32; ++c) {
-                    uint32_t v[32];
-                    tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (uint32_t)(c * 32), v);
-                    if (row < m_end) {
-#pragma unroll
-                        for (int x = 0; x < 8; ++x) {
-                            const uint32_t unit = (uint32_t)(c * 8 + x) ^ (row_local & 7u);
-                            *reinterpret_cast<uint4*>(sm + (size_t)row_local * (BN * 4) + unit * 16) =
-                                make_uint4(v[4 * x], v[4 * x + 1], v[4 * x + 2], v[4 * x + 3]);
+                                for (int x = 0; x < 4; ++x)
+                                    reinterpret_cast<uint4*>(dst)[x] = make_uint4(packed[4 * x], packed[4 * x + 1], packed[4 * x + 2], packed[4 * x + 3]);
+                            }
                         }
                     }
+                } else if (!LIN && ok && p.splits == 1 && (AR && p.ar_world > 1)) {
+                    // tensor-parallel sum in the epilogue: first push every unit of this thread's row, then
+                    // collect the peers' units (the NVLink latency of all pushes overlaps)
+                    const GemmSeg sg = p.seg[0];
+#pragma unroll 1
+                    for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll 1
+                        for (int c = 0; c < BN / 32; ++c) {
+                            uint32_t v[32];
+                            tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (uint32_t)(c * 32), v);
+                            const uint32_t col0 = n0 + c * 32;
+                            if (row >= p.m || col0 >= p.n) continue;
+#pragma unroll 1
+                            for (int x = 0; x < 8; ++x) {
+                                if (col0 + 4 * x >= p.n) break;
+                                const float mine4[4] = {__uint_as_float(v[4 * x]), __uint_as_float(v[4 * x + 1]), __uint_as_float(v[4 * x + 2]),
+                                                        __uint_as_float(v[4 * x + 3])};
+                                const uint2 mine = ar_pack<F16>(mine4);
+                                const uint64_t idx = (uint64_t)row * p.n + col0 + 4 * x, unit = idx >> 2;
+                                if (pass == 0) {
+                                    ar_push(p, ar_epoch, ar_units, unit, mine);
+                                    continue;
+                                }
+                                float a4[4];
+                                if (!ar_sum<F16>(p, ar_epoch, ar_units, unit, mine, a4)) {
+                                    atomicOr(p.status, 8u);
+                                    continue;
+                                }
+                                uint16_t h[4];
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) h[e] = epilogue_elem<F16>(a4[e], nullptr, sg.residual, idx + e);
+                                *reinterpret_cast<uint2*>(sg.out + idx) = make_uint2((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16));
+                            }
+                        }
+                    }
+                } else if (!LIN && ok && p.splits == 1) {
+#pragma unroll 1
+                    for (int c = 0; c < BN / 32; ++c) {
+                        uint32_t v[32];
+                        tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (uint32_t)(c * 32), v);
+                        const uint32_t col0 = n0 + c * 32;
+                        if (row < p.m && col0 < p.n) {
+                            uint32_t si = 0;
+                            while (si + 1 < p.nseg && col0 >= p.seg[si].col_end) ++si;
+                            const GemmSeg sg = p.seg[si];
+                            const uint64_t idx0 = (uint64_t)row * (sg.col_end - sg.col_begin) + (col0 - sg.col_begin);
+                            uint16_t* dst = sg.out + idx0;
+                            if (col0 + 32 <= sg.col_end && ((uintptr_t)dst & 15u) == 0) {
+                                uint32_t w[16];
+#pragma unroll
+                                for (int x = 0; x < 16; ++x) {
+                                    uint16_t lo = epilogue_elem<F16>(__uint_as_float(v[2 * x]), sg.table, sg.residual, idx0 + 2 * x);
+                                    uint16_t hi = epilogue_elem<F16>(__uint_as_float(v[2 * x + 1]), sg.table, sg.residual, idx0 + 2 * x + 1);
+                                    w[x] = (uint32_t)lo | ((uint32_t)hi << 16);
+                                }
+#pragma unroll
+                                for (int x = 0; x < 4; ++x)
+                                    reinterpret_cast<uint4*>(dst)[x] = make_uint4(w[4 * x], w[4 * x + 1], w[4 * x + 2], w[4 * x + 3]);
+                            } else {
+#pragma unroll
+                                for (int x = 0; x < 32; ++x)
+                                    if (col0 + x < sg.col_end) dst[x] = epilogue_elem<F16>(__uint_as_float(v[x]), sg.table, sg.residual, idx0 + x);
+                            }
+                        }
+                    }
+                } else if (ok) {
+                    // split-K: few rows go to the CTAs that add them up. More are parked in the (now idle) ring; 16-byte units of a
+                    // row are XOR-swizzled with the row number so that the 32 rows of a warp do not hit one bank
+                    const uint32_t row_local = quarter * 32 + lane;
+                    uint32_t to = 0;
+                    if (S::PUSH && row < m_end) {
+                        const uint32_t part = (split * ((15u + p.splits) / p.splits) + row_local / p.splits) * (BN * 4);
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(base + S::PUSHED + part), "r"(row_local % p.splits));
+                    }
+                    if (m0 + quarter * 32 < m_end) {  // warp-uniform: the TMEM load is a whole-warp instruction
+#pragma unroll 1
+                        for (int c = 0; c < BN / 32; ++c) {
+                            uint32_t v[32];
+                            tmem_ld32(tmem_base + ((quarter * 32u) << 16) + (uint32_t)(c * 32), v);
+                            if (S::PUSH && row < m_end) {
+#pragma unroll
+                                for (int x = 0; x < 8; ++x)
+                                    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
+                                                 ::"r"(to + (c * 8 + x) * 16), "r"(v[4 * x]), "r"(v[4 * x + 1]), "r"(v[4 * x + 2]), "r"(v[4 * x + 3]) : "memory");
+                            } else if (row < m_end) {
+#pragma unroll
+                                for (int x = 0; x < 8; ++x) {
+                                    const uint32_t unit = (uint32_t)(c * 8 + x) ^ (row_local & 7u);
+                                    *reinterpret_cast<uint4*>(sm + (size_t)row_local * (BN * 4) + unit * 16) =
+                                        make_uint4(v[4 * x], v[4 * x + 1], v[4 * x + 2], v[4 * x + 3]);
+                                }
+                            }
+                        }
+                    }
                 }
+                if (!(LIN && pushes)) break;      // the parked rows are added up below
+                __syncwarp();
+                asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+                asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
             }
+            if (ok) add_up(live != 0);
         }
     }
-    if (p.splits > 1) {
+    if (LIN && S::PUSH && p.splits > 1) {
+        if (warp < 2) {
+            __syncwarp();
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        }
+    } else if (p.splits > 1) {
         // ---- cluster reduction (all threads of all CTAs of the cluster pass both barriers) ----
         __syncwarp();  // the single-lane producer / issuer loops rejoin their warps first
+        if (S::PUSH && warp < 2) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (warp >= 2 && !*s_abort) {
             const uint32_t rank = split, S_ = p.splits, ew = warp - 2;
             const uint32_t rows_valid = min(m_end - m0, (uint32_t)BM);
-            uint32_t remote[8];
+            uint32_t remote[8];      // where the splits' parts are; pushed ones are in this CTA's own shared memory
 #pragma unroll
             for (uint32_t sidx = 0; sidx < 8; ++sidx) {
                 remote[sidx] = 0;
-                if (sidx < S_) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote[sidx]) : "r"(base), "r"(sidx));
+                if (S::PUSH) remote[sidx] = base + S::PUSHED + sidx * ((15u + S_) / S_) * (BN * 4);
+                else if (sidx < S_) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote[sidx]) : "r"(base), "r"(sidx));
             }
+            auto offset_of = [&](uint32_t rl, uint32_t u) { return S::PUSH ? rl / S_ * (BN * 4) + u * 16 : rl * (BN * 4) + ((u ^ (rl & 7u)) * 16); };
+            auto read_part = [&](uint32_t at) {
+                float4 v;
+                if (S::PUSH) asm volatile("ld.shared::cta.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+                else asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+                return v;
+            };
             if (!LIN && p.gated) {
                 // BN = 128: units 0..15 of a row are gate columns, 16..31 the matching up columns
                 const uint32_t half_n = p.n >> 1;
@@ -683,15 +760,12 @@ matmul_bf16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const uint32_t u = lane + 16 * h;
-                        const uint32_t off = rl * (BN * 4) + ((u ^ (rl & 7u)) * 16);
+                        const uint32_t off = offset_of(rl, u);
                         float4 part[8];
 #pragma unroll
                         for (uint32_t sidx = 0; sidx < 8; ++sidx) {
                             part[sidx] = make_float4(0.f, 0.f, 0.f, 0.f);
-                            if (sidx < S_)
-                                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                             : "=f"(part[sidx].x), "=f"(part[sidx].y), "=f"(part[sidx].z), "=f"(part[sidx].w)
-                                             : "r"(remote[sidx] + off));
+                            if (sidx < S_) part[sidx] = read_part(remote[sidx] + off);
                         }
                         acc[h] = part[0];
 #pragma unroll
@@ -718,15 +792,12 @@ matmul_bf16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                 const GemmSeg sg = p.seg[si];
                 const uint32_t width = sg.col_end - sg.col_begin, colseg = n0 - sg.col_begin + lane * 4;
                 for (uint32_t rl = rank + S_ * ew; rl < rows_valid; rl += S_ * 4) {
-                    const uint32_t off = rl * (BN * 4) + ((lane ^ (rl & 7u)) * 16);
+                    const uint32_t off = offset_of(rl, lane);
                     float4 part[8];
 #pragma unroll
                     for (uint32_t sidx = 0; sidx < 8; ++sidx) {
                         part[sidx] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (sidx < S_)
-                            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                         : "=f"(part[sidx].x), "=f"(part[sidx].y), "=f"(part[sidx].z), "=f"(part[sidx].w)
-                                         : "r"(remote[sidx] + off));
+                        if (sidx < S_) part[sidx] = read_part(remote[sidx] + off);
                     }
                     float4 acc = part[0];
 #pragma unroll
@@ -787,15 +858,12 @@ matmul_bf16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             for (int pass = (AR && p.ar_world > 1) ? 0 : 1; pass < 2; ++pass)
             for (uint32_t rl = rank + S_ * ew; rl < rows_valid; rl += S_ * 4) {
                 for (uint32_t u = lane; u < BN / 4; u += 32) {
-                    const uint32_t off = rl * (BN * 4) + ((u ^ (rl & 7u)) * 16);
+                    const uint32_t off = offset_of(rl, u);
                     float4 part[8];
 #pragma unroll
                     for (uint32_t sidx = 0; sidx < 8; ++sidx) {
                         part[sidx] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (sidx < S_)
-                            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                         : "=f"(part[sidx].x), "=f"(part[sidx].y), "=f"(part[sidx].z), "=f"(part[sidx].w)
-                                         : "r"(remote[sidx] + off));
+                        if (sidx < S_) part[sidx] = read_part(remote[sidx] + off);
                     }
                     float4 acc = part[0];
 #pragma unroll
@@ -840,8 +908,10 @@ matmul_bf16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             }
         }
         // nobody leaves (and frees its shared memory) while a neighbour may still read it
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (!S::PUSH) {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        }
     }
     // everyone meets here, whatever happened above, so that TMEM is always released
     __syncwarp();  // the single-lane producer / issuer loops rejoin their warps first
