@@ -13,8 +13,11 @@
 // 0.0002076. Scores need no split: products of 16-bit values are exact in f32.
 // TMEM (512 columns): S at 0 and 128, overwritten by its weights (first terms, then second terms), O at 256 and 384.
 // Bound: three products per score on the tensor core (1536 cycles a 128 x 128 tile at dim 128) against 1024 cycles of ex2.
-// 2048 rows, 32 heads over 8, dim 128, causal, bf16: one CTA per row on the CUDA cores took 48450 us, this 68 us (the tensor
-// core's share 24 us). Error against 64 bits 0.0032 in both: the output's own 16 bits.
+// What bounds it is the issuer: while it waits nothing is queued, so the next scores are issued right behind a product (one thread's
+// products execute in order; the scores' commit covers the product too) and the descriptors' words step by constants.
+// 2048 rows, 32 heads over 8, dim 128, causal, bf16: one CTA per row on the CUDA cores took 48450 us, this 58.7 us (67.6 with a wait
+// between a product and the next scores; the tensor core's share 24 us); all keys 122 -> 99.4, dim 64 108 -> 93. Error against 64 bits
+// 0.0032 in all: the output's own 16 bits. Rounding the two terms with integer operations instead of conversions: 64.4 -> 68.9.
 //
 // A weight of zero times an infinite or NaN value is NaN, and so is the sum of an infinite value's two terms: a value that is not
 // finite spoils its column of O in every row of the tile. compute_again sets that right.
@@ -74,9 +77,9 @@ constexpr float WILD = 0x1p22f;     // from here on rounding moves exponents of 
 // Columns that are not finite in a row whose sum is, and whole rows with a sum that is not or with exponents beyond WILD: scores by
 // another product, weights in f32, only the keys that a row sees, one thread a row. All threads come here, with every load and product
 // at its end; nobody leaves early, they meet after each tile. One column of 2048 rows, 32 heads over 8, dim 128, causal: 285 us instead
-// of 69 (redoing the rows one after another 124000, the general routine 48400); 12 heads x 128 rows, dim 64 19 instead of 6.7 (1580,
-// 90); 16 rows 12 instead of 5.7 (89, 9). That it can be reached costs finite inputs, in a loop that is the same, 0 to 2 % in bf16 (67.4
-// -> 68.9) and 0 to 4 % in f16 (70.0 -> 72.4), called or inlined: the registers are given out differently.
+// of 69, which is 59 by now (redoing the rows one after another 124000, the general routine 48400); 12 heads x 128 rows, dim 64 19 instead of 6.7 (1580,
+// 90); 16 rows 12 instead of 5.7 (89, 9). That it can be reached costs finite inputs, in a loop that is the same, 0 to 2 % in bf16
+// and 0 to 4 % in f16 (as measured at 67.4 and 70.0 us of this size), called or inlined: the registers are given out differently.
 template <bool F16>
 __device__ __noinline__ void compute_again(const CUtensorMap& map_k, const CUtensorMap& map_v, const RowsParams& p, uint8_t* sm, uint32_t tmem_base, uint32_t row0,
                                            uint32_t n0, uint32_t n1) {

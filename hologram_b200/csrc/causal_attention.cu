@@ -441,8 +441,10 @@ int32_t try_split(holo_b200_ctx* ctx, const HoloCausalArgs& a, bool* taken) {
 //              buffer j % 2: tcgen05.ld half a row of S, cap, exponentiate, sum, tcgen05.st the bf16 weights
 // Without a running maximum O needs no correction: it stays in TMEM from the first tile to the last.
 // TMEM (all 512 columns): S at 0 and 128, O from 256; P at 384 and 448 where vdim leaves room, else over the S it came from,
-// each key half's weights over the first half of its scores (the next scores then come behind the item's product). It is allocated after the dependency wait, and dependents are
-// released only after the allocation, so no neighbouring launch can hold columns this kernel or its predecessor waits for.
+// each key half's weights over the first half of its scores (the next scores then come behind the item's product). It is allocated
+// after the dependency wait, and dependents are released only after the allocation, so no neighbouring launch can hold columns this
+// kernel or its predecessor waits for. Bound by the hand-overs between issuer and weight warps: scores issued behind the product
+// without a wait, descriptors stepped by constants, 1531 rows, 16 heads over 4: 45.4 -> 42.4 us.
 constexpr int TILE_THREADS = 576;
 
 struct TileParams {

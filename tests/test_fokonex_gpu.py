@@ -146,6 +146,25 @@ def test_linear_adds_into_the_residual_stream(backend, dtype, m, k, n):
     assert np.abs(load(ws.read(2, m * n * 4), F32).reshape(m, n) - want).max() < 3e-5      # accumulation is f32 for both
 
 
+@pytest.mark.parametrize("bn", [64, 128])
+@pytest.mark.parametrize("splits", [1, 2, 3, 5, 7, 8])
+@pytest.mark.parametrize("m", [1, 7, 16])
+def test_linear_of_few_rows_adds_up_any_split(backend, monkeypatch, m, splits, bn):
+    """Each CTA of a split's cluster adds up every splits-th row; the parts of 7 splits take the most room. 16 rows are the tile's last."""
+    monkeypatch.setenv("HOLO_GEMM_SPLITS", str(splits))
+    monkeypatch.setenv("HOLO_GEMM_BN", str(bn))
+    k, n = 9 * 64 + 24, 200
+    rng = np.random.default_rng(m)
+    a, x = rounded(rng.standard_normal((m, k)), BF), rng.standard_normal((m, n)).astype(np.float32)
+    b = rounded(rng.standard_normal((k, n)) / np.sqrt(k), BF)
+    ws = workspace(backend, [store(a, BF), store(b, BF), x], [])
+    c = kc.LinearCall.make(kc.rb(0), kc.rb(1), [kc.LinearSeg(kc.rb(2), kc.NONE, 0, n, 0, n, 0, F32)], m, k, n, BF, residual=kc.rb(2))
+    for times in (1, 2):       # the second call adds to what the first one stored
+        backend.dispatch(kc.KernelCall.Linear(c), ws)
+        want = x + times * (a.astype(np.float64) @ b)
+        assert np.abs(load(ws.read(2, m * n * 4), F32).reshape(m, n) - want).max() < 3e-5      # f32 sums of exact products, as above
+
+
 def test_linear_refuses_what_it_cannot_do(backend):
     from hologram_b200 import BackendError
     ws = workspace(backend, [np.zeros(64 * 64, np.float32)] * 3, [])

@@ -312,3 +312,18 @@ def test_few_row_tiles_of_a_long_k_on_half_width_pairs(backend, monkeypatch, m, 
     assert norm_max_err(orc.bf16_to_f32(got), want) <= 1e-2
     monkeypatch.setenv("HOLO_GEMM_PERSISTENT", "0")
     assert np.array_equal(got, run(backend, a, b, m, k, n, act=act, residual=r))
+
+
+@pytest.mark.parametrize("bn", [64, 128])
+@pytest.mark.parametrize("splits", [2, 3, 5, 7, 8])
+@pytest.mark.parametrize("m,n,act,res", [(1, 200, 0, True), (7, 328, kc.FUSED_SILU, False), (16, 136, 0, True)])
+def test_few_rows_add_up_any_split(backend, monkeypatch, m, n, act, res, splits, bn):
+    # the parts of a K split are written to the CTA that adds them up: every splits-th row, ragged last tiles; the other kernels' tolerance
+    k = 9 * 64 + 24
+    a, b = synth(m, k, n, m + n)
+    r = orc.f32_to_bf16_rne(np.random.default_rng(1).standard_normal(m * n, dtype=np.float32)) if res else None
+    monkeypatch.setenv("HOLO_GEMM_SPLITS", str(splits))
+    monkeypatch.setenv("HOLO_GEMM_BN", str(bn))
+    got = run(backend, a, b, m, k, n, act=act, residual=r)
+    want = orc.bf16_to_f32(orc.matmul(a, b, m, k, n, BF, act=act, residual=r))
+    assert norm_max_err(orc.bf16_to_f32(got), want) <= 1e-2
