@@ -1485,9 +1485,11 @@ int32_t launch_persistent(holo_b200_ctx* ctx, const CUtensorMap& ma, const CUten
 // walked by one CTA per SM (WALK), or a CTA per tile (tile_choice). What each takes, in ns, fitted to 249 shapes of 130 .. 4096 rows, each
 // timed with all four: a start and, per round of items, an epilogue and what a k-block costs. Per SM and k-block a pair reads 32 KiB for
 // 256 x 256 and 24 KiB for 256 x 128, CTAs with 128 x 64 tiles read 24 KiB each, two of them on an SM: that is why few tiles of a
-// long k do better as halves on pairs (1024 x 8192 x 2048 43.7 -> 36.5 us, 446 x 2536 x 3440 31 -> 20, 1024 x 2048 x 2048 15.5 -> 14.8), and one
-// round of whole tiles better than two of CTAs (2048 x 10240 x 2048 75 -> 63). The choice was 1 % above the best of the four on average
-// (12.9 us, geometric mean; without halves and with pairs from a full round on only, 13.5); 1.15 where the estimate misled it, hence the margins.
+// long k do better as halves on pairs (1024 x 8192 x 2048 43.7 -> 36.5 us, 446 x 2536 x 3440 31 -> 20, 1024 x 2048 x 2048 15.5 -> 14.8), and
+// one round of whole tiles better than two of CTAs (2048 x 10240 x 2048 75 -> 63). The choice was 1 % above the best of the four on
+// average (12.9 us, geometric mean; without halves and with pairs from a full round on only, 13.5); 1.15 where the estimate misled it,
+// hence the margins. Against a CTA per tile pairs have to gain 12 % of the estimate: between other kernels they lose what those gain by
+// starting early (292 x 2048 x 512 in a bf16 encoder 17 -> 21 us; its block of 292 rows 180 us, 183 without the margin, 175 with it).
 enum BigKernel { CTA_PER_TILE, WALK, PAIRS, HALF_PAIRS };
 inline BigKernel big_choice(const holo_b200_ctx* ctx, uint32_t m, uint32_t n, uint32_t kblocks) {
     const uint64_t sms = (uint64_t)ctx->sm_count, pairs = sms / 2, kb = kblocks;
@@ -1514,8 +1516,10 @@ inline BigKernel big_choice(const holo_b200_ctx* ctx, uint32_t m, uint32_t n, ui
         if (atoi(e) == 0) return CTA_PER_TILE;
     if (const char* e = getenv("HOLO_GEMM_PAIR"))
         if (atoi(e) == 0) return ptiles >= sms ? WALK : CTA_PER_TILE;
-    if (best != PAIRS && whole_ns < best_ns) best = PAIRS, best_ns = whole_ns;
-    return half_ns < best_ns ? HALF_PAIRS : best;
+    // one CTA per tile starts beside the kernel before it, pairs with their whole shared memory do not
+    const uint64_t of = best == CTA_PER_TILE ? 28 : 25;
+    if (best != PAIRS && whole_ns * of / 25 < best_ns) best = PAIRS, best_ns = whole_ns * of / 25;
+    return half_ns * of / 25 < best_ns ? HALF_PAIRS : best;
 }
 
 // Tile width and K split of the one-tile-per-CTA kernel. Compute-bound shapes (many row tiles) take 128-wide tiles, no split.

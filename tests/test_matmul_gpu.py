@@ -300,7 +300,7 @@ def test_persistent_tile_kernels_within_tolerance(backend, monkeypatch, m, k, n,
     assert np.array_equal(outs["pair"], outs["classic"]) and np.array_equal(outs["persistent"], outs["classic"])
 
 
-@pytest.mark.parametrize("m,k,n,act,res", [(257, 4160, 392, 0, False), (1000, 2544, 1936, kc.FUSED_SILU, False), (130, 8000, 264, 0, True), (300, 2000, 136, 0, False),
+@pytest.mark.parametrize("m,k,n,act,res", [(257, 4160, 392, 0, False), (1000, 2544, 1936, kc.FUSED_SILU, False), (1000, 2496, 1928, 0, False), (900, 2600, 1936, 0, True), (130, 8000, 264, 0, True), (300, 2000, 136, 0, False),
                                            (300, 2056, 136, 0, False), (300, 2120, 136, 0, False), (260, 1536, 2056, 0, False), (513, 1984, 640, 0, True)])
 def test_few_row_tiles_of_a_long_k_on_half_width_pairs(backend, monkeypatch, m, k, n, act, res):
     # fewer tiles than pairs of SMs: 256 x 128 items, three k-blocks a stage (remainders of 0, 1 and 2 among these), ragged last tiles.
