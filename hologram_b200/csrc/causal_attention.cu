@@ -133,13 +133,13 @@ __device__ __forceinline__ float2 capped_exp_small(uint64_t s, uint64_t c0, uint
 // last CTA of a (kv head, row tile) to count in adds the partials in split order; nobody waits.
 // At short caches it is bound by latency. Where one tile for each warp covers the cache (STAGES 1) there is no ring: 75 KiB of
 // shared memory in place of 209 let its CTAs start beside the ones of the product before it, which runs for 10 us more. They bring
-// their part of the cache into L2 meanwhile, and a warp's tile does not depend on the position. Every division that gives a place
-// stands before the wait, the queries are requested before the position is known, and in the last CTA a thread has twelve
-// splits' parts of its cells and of their row's sum on their way at a time and finishes them itself. 16 heads over 4, dim 128, on
-// the critical path of a step: 1532 keys 12 -> 7.5 us (of it 1.9 keys and values, 1.0 products and weights, 0.8 warps, 1.0
-// arrival, 0.9 parts, 0.6 result); alone 10.3 -> 7.5, 8192 rows of cache (three stages) 13.0 -> 10.8; four rows 15.9 -> 10.0; dim
-// 256 with eight rows 45.9 -> 19.0. Requesting by the position read before the wait, or going through the code once before it,
-// changed nothing.
+// their part of the cache into L2 meanwhile. The keys are shared out as with a ring, so the sums are the same bits wherever the ring has
+// room for eight warps as well (not at dim 256, say). Every division that gives a place stands before the wait, the queries are
+// requested before the position is known, and in the last CTA a thread has twelve splits' parts of its cells and of their row's sum on
+// their way at a time and finishes them itself. 16 heads over 4, dim 128, on the critical path of a step: 1532 keys 12 -> 7.5 us (of
+// it 1.9 keys and values, 1.0 products and weights, 0.8 warps, 1.0 arrival, 0.9 parts, 0.6 result); alone 10.3 -> 7.5, 8192 rows of
+// cache (three stages) 13.0 -> 10.8; four rows 15.9 -> 10.0; dim 256 with eight rows 45.9 -> 19.0. Requesting by the position read
+// before the wait, or going through the code once before it, changed nothing.
 constexpr uint32_t SPLIT_SLOTS = 1024, SPLIT_SLOT_FLOATS = 16 * 257;
 
 struct SplitParams {
@@ -167,17 +167,31 @@ causal_attention_split_kernel(const SplitParams p) {
     // the last position any row of this tile sees
     const uint32_t last_row = min((z * 16 + 15) / p.group, a.rows - 1);
     auto visible_at = [&](uint32_t at) { return (uint32_t)min((uint64_t)at + last_row + 1, (uint64_t)a.cache_rows); };
+    // The tiles of split c: an even share, with or without a ring, so that a cell's sum groups its keys the same way in both
+    struct Share {
+        uint32_t used, begin, end;
+    };
+    auto share_at = [&](uint32_t seen) {
+        const uint32_t tiles = (seen + 15) / 16, used = min(p.splits, (tiles + nwarps - 1) / nwarps);
+        if (STAGES == 1) return Share{used, tiles * split / used, tiles * (split + 1) / used};     // at most 8 tiles a split and a split an SM
+        return Share{used, (uint32_t)((uint64_t)tiles * split / used), (uint32_t)((uint64_t)tiles * (split + 1) / used)};
+    };
     // The position before the wait is a guess: the kernel ahead, or one ahead of it, may still write it. It only chooses which
-    // rows of the cache to bring into L2 meanwhile, and is read past L1 so that the read after the wait cannot meet it there.
+    // rows of the cache to bring into L2 meanwhile, and is read past L1 so that the read after the wait cannot meet it there. Where it
+    // was right, the share needs no division after the wait.
     auto read_pos = [&] {
         uint32_t v;
         asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.pos) : "memory");
         return v;
     };
+    uint32_t guess = 0;
+    Share share = {};
     if (STAGES == 1) {
-        const uint32_t guess = visible_at(read_pos()), from = split * nwarps * 16, to = min(guess, from + nwarps * 16);
+        guess = read_pos();
+        share = share_at(visible_at(guess));
+        const uint32_t to = split < share.used ? min(visible_at(guess), share.end * 16) : 0;
         const uint32_t klines = (a.dim * 2 + 127) / 128, vlines = (a.vdim * 2 + 127) / 128;
-        for (uint32_t key = from + threadIdx.x; key < to; key += blockDim.x) {
+        for (uint32_t key = share.begin * 16 + threadIdx.x; key < to; key += blockDim.x) {
             for (uint32_t i = 0; i < klines; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(kbase + (uint64_t)key * kv_ld + 64 * i));
             for (uint32_t i = 0; i < vlines; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(vbase + (uint64_t)key * vv_ld + 64 * i));
         }
@@ -202,14 +216,12 @@ causal_attention_split_kernel(const SplitParams p) {
     for (uint32_t i = threadIdx.x + blockDim.x; i < 16 * kvec; i += blockDim.x) request_q(i / kvec, i % kvec, (z * 16 + i / kvec) / p.group, (z * 16 + i / kvec) % p.group);
     asm volatile("cp.async.commit_group;" ::: "memory");
     const uint32_t visible = visible_at(pos);
-    const uint32_t tiles = (visible + 15) / 16;
-    const uint32_t used = min(p.splits, (tiles + nwarps - 1) / nwarps);
+    if (STAGES > 1 || pos != guess) share = share_at(visible);
+    const uint32_t used = share.used, t_begin = share.begin, t_end = share.end;
     if (split >= used) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         return;
     }
-    const uint32_t t_begin = STAGES == 1 ? split * nwarps : (uint32_t)((uint64_t)tiles * split / used);
-    const uint32_t t_end = STAGES == 1 ? min(tiles, t_begin + nwarps) : (uint32_t)((uint64_t)tiles * (split + 1) / used);
     auto load_rows = [&](uint32_t dst, uint32_t pitch, const __nv_bfloat16* src, uint32_t ld, uint32_t first, uint32_t vecs, uint32_t r, uint32_t c, uint32_t dr, uint32_t dc) {
 #pragma unroll 4
         while (r < 16) {

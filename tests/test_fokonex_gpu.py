@@ -322,6 +322,19 @@ def test_attention_of_few_rows_around_the_longest_cache_without_a_ring(backend, 
         assert np.abs(got - want).max() / np.abs(want).max() < 1e-2, first      # weights and results in bf16, as above
 
 
+@pytest.mark.parametrize("shape", [(1, 8, 8, 32, 32), (3, 12, 4, 48, 80), (2, 8, 2, 80, 128), (1, 16, 4, 128, 128), (5, 8, 2, 64, 176)], ids=lambda s: "-".join(map(str, s)))
+def test_attention_without_a_ring_adds_up_in_the_ring_s_order(backend, shape):
+    """The same keys in a cache of one row more, which takes the ring: the splits have the same keys, so the bits are the same."""
+    rows, heads, groups, dim, vdim = shape
+    splits = torch.cuda.get_device_properties(0).multi_processor_count // (-(-rows * heads // groups // 16) * groups)
+    cache = splits * 8 * 16
+    q, k, v, sinks = random_attention(rows, heads, groups, dim, vdim, cache, seed=rows + dim)
+    for first in (0, 129 - rows, 150, cache // 2 + 1, cache - 40, cache - rows):
+        seen = first + rows
+        got = [run_attention(backend, q, k[:seen], v[:seen], first, dim ** -0.5, 25.0, 0.3, 16, sinks, BF, cache + extra) for extra in (0, 1)]
+        assert np.array_equal(got[0], got[1]), first
+
+
 # ---- whole models ----
 TOL = {"float32": 2e-5, "bfloat16": 4e-2}
 
