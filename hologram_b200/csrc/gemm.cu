@@ -101,7 +101,7 @@ int32_t holo_launch_matmul_multi(holo_b200_ctx* ctx, const void* a, const void* 
     if (cell_path) return holo_launch_matmul_cell(ctx, a, b, out, table, segs[0].fused_act ? lut_id_of_fused(segs[0].fused_act) : -1, residual, m, k, n, dtype, 0);
     const uint32_t kblocks = (k + BK - 1) / BK, mtiles = (m + BM - 1) / BM;
     {
-        BigKernel big = big_choice(ctx, m, n, kblocks);
+        BigKernel big = big_choice((uint32_t)ctx->sm_count, m, n, kblocks, 1);
         if (gated || (segs[0].all_reduce && ctx->tp_world > 1)) big = CTA_PER_TILE;
         if (big != CTA_PER_TILE) {
             GemmParams p;
@@ -124,7 +124,7 @@ int32_t holo_launch_matmul_multi(holo_b200_ctx* ctx, const void* a, const void* 
     }
     int bn;
     uint32_t splits;
-    tile_choice(ctx, m, n, kblocks, &bn, &splits);
+    tile_choice((uint32_t)ctx->sm_count, m, n, kblocks, &bn, &splits);
     const uint32_t tiles128 = mtiles * ((n + 127) / 128);
     if (const char* e = getenv("HOLO_GEMM_BN")) bn = atoi(e) == 64 ? 64 : atoi(e) == 256 ? 256 : 128;
     if (gated && bn != 128) {   // the gate / up pairing is per 128-wide tile

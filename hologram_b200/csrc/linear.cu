@@ -219,29 +219,26 @@ int32_t holo_launch_linear(holo_b200_ctx* ctx, const HoloLinearArgs& a) {
     HOLO_TRY(make_map_2d(&mb, a.b, a.n, (uint64_t)a.k * (a.tiles ? a.experts : 1), 64, BK));
     // rows A has: the matrix's own, a ring's, or the ones all tiles of a group share
     const uint64_t a_rows = a.a_pos ? a.a_rows : a.a_shared ? a.a_shared : a.m;
-    BigKernel big = big_choice(ctx, a.m, a.n, kblocks);
-    if (a.tiles) {      // neighbouring row tiles may belong to different experts: no pairs
-        const bool walk = a.tile_rows == (uint32_t)BM && !a.a_shared && (uint64_t)mtiles * ((a.n + PBN - 1) / PBN) >= (uint64_t)ctx->sm_count;
+    const uint32_t sms = (uint32_t)ctx->sm_count, gtiles = a.tiles ? a.m / a.tile_rows : 0;
+    int bn;
+    uint32_t splits;
+    BigKernel big;
+    if (a.tiles) {
+        // a group is weight streaming like one product as wide as all its tiles together
+        tile_choice(sms, a.tile_rows, a.n * gtiles, kblocks, &bn, &splits);
+        // neighbouring row tiles may belong to different experts: no pairs
+        const bool walk = a.tile_rows == (uint32_t)BM && !a.a_shared && (uint64_t)mtiles * ((a.n + PBN - 1) / PBN) >= (uint64_t)sms;
         const char* e = getenv("HOLO_GEMM_PERSISTENT");
         big = walk && mtiles >= 2 && !(e && atoi(e) == 0) ? WALK : CTA_PER_TILE;
+    } else {
+        linear_tile_choice(sms, a.m, a.n, kblocks, &bn, &splits);
+        big = big_choice(sms, a.m, a.n, kblocks, splits);
     }
     if (big != CTA_PER_TILE) {
         p.box_m = BM;
         HOLO_TRY(make_map_2d(&ma, a.a, a.lda, a_rows, BK, BM));
         return big == PAIRS ? launch_pair<false, true, false>(ctx, ma, mb, p) : big == HALF_PAIRS ? launch_pair<false, true, true>(ctx, ma, mb, p)
                                                                                                   : launch_persistent<false, true>(ctx, ma, mb, p);
-    }
-    int bn;
-    uint32_t splits;
-    const uint32_t gtiles = a.tiles ? a.m / a.tile_rows : 0;
-    // a group is weight streaming like one product as wide as all its tiles together
-    if (a.tiles) tile_choice(ctx, a.tile_rows, a.n * gtiles, kblocks, &bn, &splits);
-    else tile_choice(ctx, a.m, a.n, kblocks, &bn, &splits);
-    if (!a.tiles && mtiles > 1 && splits == 1) {      // many rows, few columns (a router): K slices fill the chip
-        const uint32_t tiles = mtiles * ((a.n + bn - 1) / bn);
-        splits = (uint32_t)ctx->sm_count / tiles;
-        if (splits > kblocks / 4) splits = kblocks / 4;
-        if (splits < 1) splits = 1;
     }
     if (const char* e = getenv("HOLO_GEMM_BN")) bn = atoi(e) == 64 ? 64 : 128;
     if (const char* e = getenv("HOLO_GEMM_SPLITS")) splits = (uint32_t)atoi(e) > 0 ? (uint32_t)atoi(e) : 1;
