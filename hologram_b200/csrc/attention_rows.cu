@@ -13,8 +13,8 @@
 // 0.0002076. Scores need no split: products of 16-bit values are exact in f32.
 // TMEM (512 columns): S at 0 and 128, overwritten by its weights (first terms, then second terms), O at 256 and 384.
 // Bound: three products per score on the tensor core (1536 cycles a 128 x 128 tile at dim 128) against 1024 cycles of ex2.
-// What bounds it is the issuer: while it waits nothing is queued, so the next scores are issued right behind a product (one thread's
-// products execute in order; the scores' commit covers the product too) and the descriptors' words step by constants.
+// What bounds it is the issuer: while it waits nothing is queued, so the next scores are issued right behind a product (on what that rests
+// stands at product_ss; the scores' commit covers the product too) and the descriptors' words step by constants.
 // 2048 rows, 32 heads over 8, dim 128, causal, bf16: one CTA per row on the CUDA cores took 48450 us, this 58.7 us (67.6 with a wait
 // between a product and the next scores; the tensor core's share 24 us); all keys 122 -> 99.4, dim 64 108 -> 93. Error against 64 bits
 // 0.0032 in all: the output's own 16 bits. Rounding the two terms with integer operations instead of conversions: 64.4 -> 68.9.
@@ -362,7 +362,7 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                         for (uint32_t k = 0; k < steps; ++k) product_ts(d, tmem_p + 64 + k * 8, dv + 128 * k, high_v, idesc_o, 1);
                     }
                     umma_commit(bar_pv + 8 * q);
-                    // the next scores go where the weights are; one thread's products execute in order, so nothing waits for the last one
+                    // the next scores go where the weights are, behind the product that reads them (see product_ss)
                     if (next < n) scores(q, next);
                 }
                 if (!ok) break;

@@ -74,6 +74,11 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
 }
 // The same products with descriptors in two words: steps of a tile only change the lower one, by constants, and the one thread that issues
 // them has little time for each.
+// The attention kernels issue a tile's next scores right behind the product that still reads the weights they overwrite. The PTX ISA
+// promises issue order for products of one accumulator and one shape only; these differ in both. That the tensor core takes all
+// products of a thread in the order of their issue is how this chip is seen to behave, not what is documented: published attention kernels for it
+// overwrite weights in the same way, and the tests that repeat long sequences bit for bit (test_attention_gpu.py, test_fokonex_gpu.py)
+// and those against 64 bits would show a product that overtakes another. Waiting for the product instead costs 9 us of 68 (attention_rows.cu).
 __device__ __forceinline__ void product_ss(uint32_t tmem_d, uint32_t a, uint32_t a_high, uint32_t b, uint32_t b_high, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n.reg .pred p;\n.reg .b64 x, y;\nmov.b64 x, {%1, %2};\nmov.b64 y, {%3, %4};\nsetp.ne.b32 p, %6, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %5, p;\n}\n"

@@ -609,7 +609,7 @@ causal_attention_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __
                     umma_commit(bar_v_empty + 8 * vs);
                     if (++vs == p.vstages) vs = 0, vphase ^= 1;
                 }
-                if (alias && i + 2 < items) ok = scores(i + 2);      // behind the product that reads the weights there: one thread's products execute in order
+                if (alias && i + 2 < items) ok = scores(i + 2);      // behind the product that reads the weights there (see product_ss)
             }
             if (ok) umma_commit(bar_o);
         }

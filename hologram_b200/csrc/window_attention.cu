@@ -583,7 +583,7 @@ window_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                         umma_commit(bar_v_empty + 8 * vs);
                         if (++vs == p.vslots) vs = 0, vphase ^= 1;
                     }
-                    if (i + 1 < ntiles) ok = scores(q);
+                    if (i + 1 < ntiles) ok = scores(q);      // behind the product that reads the weights there (see product_ss)
                 }
             }
         }

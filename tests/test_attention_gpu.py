@@ -584,6 +584,31 @@ def device_tensors(shapes, dtype, seed=5):
     return [torch.randn(s, generator=g, device="cuda").to({F32: torch.float32, BF: torch.bfloat16, kc.DTYPE_F16: torch.float16}[dtype]) for s in shapes]
 
 
+@pytest.mark.parametrize("dtype", [BF, kc.DTYPE_F16])
+@pytest.mark.parametrize("d", [64, 80, 128])
+@pytest.mark.parametrize("causal", [True, False])
+def test_long_sequences_repeat_their_bits(d, dtype, causal):
+    # a tile's next scores are issued behind the product that still reads the weights they overwrite: a product that was overtaken, once in
+    # forty calls of 16 heads x 12 tiles x 12 tiles, would give other bits
+    import torch
+    b, h, kv, s = 1, 16, 4, 1500
+    be, stream = hb.B200Backend(0), torch.cuda.Stream()
+    be.set_stream(stream.cuda_stream)
+    x = device_tensors([(b, h, s, d), (b, kv, s, d), (b, kv, s, d)], dtype)
+    out = torch.zeros((40,) + tuple(x[0].shape), dtype=x[0].dtype, device="cuda")
+    torch.cuda.synchronize()
+    for o in out:
+        ws = hb.DeviceWorkspace(be, 4)
+        for i, t in enumerate(x + [o]):
+            ws.bind(i, t.data_ptr(), t.numel() * t.element_size())
+        be.dispatch(kc.KernelCall.Attention(kc.AttentionCall(*[kc.rb(i) for i in range(4)], b, h, s, d, kv, int(causal), 0, dtype)), ws)
+        ws.close()
+    stream.synchronize()
+    be.close()
+    bits = out.view(torch.int16)
+    assert bits[0].any() and (bits == bits[0]).all()
+
+
 @pytest.mark.parametrize("b,h,kv,past,d,dtype", [(64, 32, 32, 3, 64, F32), (64, 32, 32, 7, 64, BF), (256, 12, 12, 3, 128, BF), (32, 12, 12, 3, 64, kc.DTYPE_F16),
                                                  (64, 32, 32, 23, 64, F32), (16, 32, 8, 3, 64, F32), (1, 12, 2, 3, 128, F32)])
 def test_one_row_of_many_short_caches_takes_the_quicker_route(monkeypatch, b, h, kv, past, d, dtype):

@@ -335,6 +335,20 @@ def test_attention_without_a_ring_adds_up_in_the_ring_s_order(backend, shape):
         assert np.array_equal(got[0], got[1]), first
 
 
+@pytest.mark.parametrize("tiles", [1, 2])
+@pytest.mark.parametrize("dim,vdim", [(64, 64), (64, 80), (128, 128), (256, 256)])
+def test_attention_of_many_rows_repeats_its_bits(backend, monkeypatch, dim, vdim, tiles):
+    """Where the weights lie over their scores the next scores are issued behind the product that still reads them: an overtaken product
+    would give other bits."""
+    monkeypatch.setenv("HOLO_CAUSAL_QUERY_TILES", str(tiles))
+    q, k, v, sinks = random_attention(700, 8, 2, dim, vdim, 1500, seed=dim + vdim)
+    args = (q, k, v, 800, dim ** -0.5, 20.0, 0.2, 64, sinks, BF)
+    first = run_attention(backend, *args)
+    assert np.isfinite(first).all()
+    for _ in range(20):
+        assert np.array_equal(run_attention(backend, *args), first)
+
+
 # ---- whole models ----
 TOL = {"float32": 2e-5, "bfloat16": 4e-2}
 
