@@ -146,6 +146,20 @@ def test_linear_adds_into_the_residual_stream(backend, dtype, m, k, n):
     assert np.abs(load(ws.read(2, m * n * 4), F32).reshape(m, n) - want).max() < 3e-5      # accumulation is f32 for both
 
 
+@pytest.mark.parametrize("pairs", ["", "2"], ids=["all-pairs", "two-pairs"])
+@pytest.mark.parametrize("kernel", ["tile", "walk", "pairs", "halves"])
+def test_linear_on_every_kernel(backend, monkeypatch, kernel, pairs):
+    """Segments with their own k offset, pitch and place in a cache, and the residual stream (ragged n; a served prompt's output product; few
+    columns of a long k, which a CTA per tile splits): two pairs walk several items each."""
+    monkeypatch.setenv("HOLO_GEMM_KERNEL", kernel)
+    if pairs:
+        monkeypatch.setenv("HOLO_GEMM_PAIR_GRID", pairs)
+    for m, w, widths, up in ((300, 320, (256, 64, 64), 640), (513, 456, (96, 33, 40), 1000)):
+        test_linear_segments(backend, BF, m, w, widths, up)
+    for m, k, n in ((200, 264, 100), (1024, 2048, 1344), (257, 2120, 392), (200, 2056, 264)):
+        test_linear_adds_into_the_residual_stream(backend, BF, m, k, n)
+
+
 @pytest.mark.parametrize("bn", [64, 128])
 @pytest.mark.parametrize("splits", [1, 2, 3, 5, 7, 8])
 @pytest.mark.parametrize("m", [1, 7, 16])

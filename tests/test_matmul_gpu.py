@@ -280,8 +280,8 @@ def test_session_forms_the_f32_triple_at_load(backend):
 @pytest.mark.parametrize("m,k,n,act,res", [(4096, 256, 2560, 0, False), (2500, 320, 2320, kc.FUSED_SILU, False), (2304, 192, 2304, 0, True),
                                            (1333, 128, 8200, 0, False)])
 def test_persistent_tile_kernels_within_tolerance(backend, monkeypatch, m, k, n, act, res):
-    # shapes with at least one 256 x 256 tile per SM pair take the CTA-pair kernel (tcgen05 cta_group::2), shapes with at
-    # least one 128 x 256 tile per SM the one-CTA persistent kernel; ragged edges in both directions, fused epilogues.
+    # shapes of one 128 x 256 tile per SM and more: the CTA-pair kernel (tcgen05 cta_group::2) by its estimated time, the one-CTA
+    # persistent kernel without it; ragged edges in both directions, fused epilogues.
     # Both must agree with the CPU chain within the tensor-core tolerance, and with each other and with the
     # one-tile-per-CTA kernel bit for bit (same k order per cell: the accumulation order inside one MMA chain is fixed).
     a, b = synth(m, k, n, m + n)
@@ -300,18 +300,45 @@ def test_persistent_tile_kernels_within_tolerance(backend, monkeypatch, m, k, n,
     assert np.array_equal(outs["pair"], outs["classic"]) and np.array_equal(outs["persistent"], outs["classic"])
 
 
+@pytest.mark.parametrize("pairs", ["", "2"], ids=["all-pairs", "two-pairs"])
+@pytest.mark.parametrize("kernel", ["halves", "pairs"])
 @pytest.mark.parametrize("m,k,n,act,res", [(257, 4160, 392, 0, False), (1000, 2544, 1936, kc.FUSED_SILU, False), (1000, 2496, 1928, 0, False), (900, 2600, 1936, 0, True), (130, 8000, 264, 0, True), (300, 2000, 136, 0, False),
-                                           (300, 2056, 136, 0, False), (300, 2120, 136, 0, False), (260, 1536, 2056, 0, False), (513, 1984, 640, 0, True)])
-def test_few_row_tiles_of_a_long_k_on_half_width_pairs(backend, monkeypatch, m, k, n, act, res):
-    # fewer tiles than pairs of SMs: 256 x 128 items, three k-blocks a stage (remainders of 0, 1 and 2 among these), ragged last tiles.
+                                           (300, 2056, 136, 0, False), (300, 2120, 136, 0, False), (260, 1536, 2056, 0, False), (513, 1984, 640, 0, True), (129, 64, 8200, 0, False)])
+def test_few_row_tiles_of_a_long_k_on_pairs(backend, monkeypatch, m, k, n, act, res, kernel, pairs):
+    # 256 x 128 and 256 x 256 items, three or two k-blocks a stage (remainders of 0, 1 and 2 among these), ragged last tiles, some with no
+    # column for the pair's second CTA. Two pairs walk up to 33 items each: ring phases and accumulator buffers carry over from item to item.
+    # The kernel is named, so that no rule can take these shapes elsewhere.
     # The tolerance is the other tensor-core kernels'; the k order per cell is theirs, so the bits are too.
     a, b = synth(m, k, n, m + n)
     r = orc.f32_to_bf16_rne(np.random.default_rng(1).standard_normal(m * n, dtype=np.float32)) if res else None
+    monkeypatch.setenv("HOLO_GEMM_KERNEL", kernel)
+    if pairs:
+        monkeypatch.setenv("HOLO_GEMM_PAIR_GRID", pairs)
     got = run(backend, a, b, m, k, n, act=act, residual=r)
     want = orc.bf16_to_f32(orc.matmul(a, b, m, k, n, BF, act=act, residual=r))
     assert norm_max_err(orc.bf16_to_f32(got), want) <= 1e-2
-    monkeypatch.setenv("HOLO_GEMM_PERSISTENT", "0")
+    monkeypatch.setenv("HOLO_GEMM_KERNEL", "tile")
     assert np.array_equal(got, run(backend, a, b, m, k, n, act=act, residual=r))
+
+
+@pytest.mark.parametrize("m,k,n", [(2790, 2048, 1648), (898, 448, 4672)])
+def test_several_rounds_of_half_width_items(backend, monkeypatch, m, k, n):
+    # more 256 x 128 items than pairs of SMs, as the rule itself chooses them; one or two k-blocks are left over in the last stage
+    a, b = synth(m, k, n, m + n)
+    monkeypatch.setenv("HOLO_GEMM_KERNEL", "halves")
+    got = run(backend, a, b, m, k, n)
+    monkeypatch.setenv("HOLO_GEMM_KERNEL", "tile")
+    assert np.array_equal(got, run(backend, a, b, m, k, n))
+
+
+@pytest.mark.parametrize("pairs", ["", "2"], ids=["all-pairs", "two-pairs"])
+@pytest.mark.parametrize("kernel", ["walk", "pairs", "halves"])
+@pytest.mark.parametrize("m,k,n", [(300, 456, 200), (520, 1032, 648)])
+def test_f16_products_on_every_kernel(backend, monkeypatch, m, k, n, kernel, pairs):
+    monkeypatch.setenv("HOLO_GEMM_KERNEL", kernel)
+    if pairs:
+        monkeypatch.setenv("HOLO_GEMM_PAIR_GRID", pairs)
+    test_f16_matmul(backend, m, k, n)
 
 
 @pytest.mark.parametrize("bn", [64, 128])

@@ -124,7 +124,7 @@ def test_linear_rotates_appends_to_a_ring_and_activates(backend, dtype, rows):
 @pytest.mark.parametrize("dtype", [F32, BF])
 @pytest.mark.parametrize("m,n,pos", [(128, 64, 0), (256, 64, 300), (384, 64, 1000), (384, 4096, 700), (640, 12288, 700)])
 def test_linear_over_a_window_of_a_ring(backend, dtype, m, n, pos):
-    """Rows of A come from a ring, starting a given distance before the position (all three tensor-core kernels)."""
+    """Rows of A come from a ring, starting a given distance before the position (each tensor-core kernel: below)."""
     rng = np.random.default_rng(m)
     ring, lda, k, back = 512, 96, 80, 150
     es = 2 if dtype == BF else 4
@@ -136,6 +136,15 @@ def test_linear_over_a_window_of_a_ring(backend, dtype, m, n, pos):
     start = max(0, pos - back) // 128 * 128
     want = a[(start + np.arange(m)) % ring, :k].astype(np.float64) @ b
     close(load(ws.read(rb(3), m * n * es), dtype).reshape(m, n), want, dtype)
+
+
+@pytest.mark.parametrize("kernel", ["tile", "walk", "pairs", "halves"])
+def test_linear_of_many_rows_on_every_kernel(backend, monkeypatch, kernel):
+    monkeypatch.setenv("HOLO_GEMM_KERNEL", kernel)
+    monkeypatch.setenv("HOLO_GEMM_PAIR_GRID", "2")      # several items a pair
+    test_linear_rotates_appends_to_a_ring_and_activates(backend, BF, 300)
+    for m, n, pos in ((256, 64, 300), (384, 64, 1000), (384, 4096, 700)):
+        test_linear_over_a_window_of_a_ring(backend, BF, m, n, pos)
 
 
 @pytest.mark.parametrize("dtype", [F32, BF])
