@@ -512,8 +512,8 @@ def workload_matmul(be, torch, rank, args, skinny=False):
         "launches_per_step": 1,
         "roofline": ({"bound": "hbm", "bytes_per_launch": nbytes, "kernel": "matmul_bf16_umma_kernel", "traffic": None} if skinny else
                      {"bound": "tensor", "flops_per_launch": flops, "kernel": "matmul_umma_pair_kernel" if (m >= 256 and n >= 256 and -(-m // 256) * -(-n // 256) >= 74) else "matmul_bf16_umma_kernel",
-                      "traffic": 82_627_072 if (m, k, n) == (4096, 4096, 4096) else None,
-                      "traffic_note": "ncu, profiles/matmul_bf16_umma_kernel.md: 69.58 MB read + 13.05 MB written inside the kernel window"}),
+                      "traffic": 82_650_880 if (m, k, n) == (4096, 4096, 4096) else None,
+                      "traffic_note": "ncu, profiles/matmul_bf16_umma_kernel.md: 69.45 MB read + 13.20 MB written inside the kernel window"}),
         "h2d": 2 * (m * k + k * n), "d2h": 2 * m * n,
         "cpu_baseline": cpu_baseline, "extra": burst,
         "config": {"workload": f"config[2]: bf16 matmul M={m} K={k} N={n}, f32 accumulation, bf16 output, A,B ~ N(0, 1/K)",

@@ -131,8 +131,8 @@ __device__ __forceinline__ float2 capped_exp_small(uint64_t s, uint64_t c0, uint
 // them. Warp w of split c takes 16-key tiles w, w + W, ... of the split's range through a private ring of STAGES tiles
 // (no block-wide synchronisation in the loop). Warps merge through shared memory, splits through a partial buffer: the
 // last CTA of a (kv head, row tile) to count in adds the partials in split order; nobody waits.
-// At short caches it is bound by latency. Where one tile for each warp covers the cache (STAGES 1) there is no ring: 75 KiB of
-// shared memory in place of 209 let its CTAs start beside the ones of the product before it, which runs for 10 us more. They bring
+// At short caches it is bound by latency. Where one tile for each warp covers the cache (STAGES 1) there is no ring: 72 KiB of
+// shared memory in place of 208 let its CTAs start beside the ones of the product before it, which runs for 10 us more. They bring
 // their part of the cache into L2 meanwhile. The keys are shared out as with a ring, so the sums are the same bits wherever the ring has
 // room for eight warps as well (not at dim 256, say). Every division that gives a place stands before the wait, the queries are
 // requested before the position is known, and in the last CTA a thread has twelve splits' parts of its cells and of their row's sum on

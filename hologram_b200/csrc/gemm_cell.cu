@@ -7,7 +7,8 @@
 // equally many. One thread keeps TM x TN cells in registers; tiles of A and B (BK deep, as f32) pass through a ring in shared
 // memory, filled by cp.async (f32) or through registers (16-bit, widened once per tile instead of once per cell); the next
 // depths' operands are read from shared memory while these are multiplied. What is left is reads of shared memory (8 bytes
-// per lane and wavefront at most: a 4 x 4 thread needs as many cycles for them as for its multiply-adds) and their latency.
+// per lane and wavefront at most: 2.0 cycles for a warp's 16-byte read in both patterns below, 4.0 where no two lanes share an address. A 4 x 4
+// thread needs as many cycles for them as for its multiply-adds, a 2 x 4 thread 1.5 times as many) and their latency.
 // One thread per cell, before: 500 x 1000 x 771 f32 148 us, now 36 (21 TFLOP/s); 381 x 3072 x 768 462 us, now 81;
 // 1000 x 2048 x 2048 now 209 (40 TFLOP/s).
 #include "common.h"
