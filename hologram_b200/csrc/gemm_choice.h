@@ -16,7 +16,7 @@ constexpr int BM = 128, BK = 64, PBN = 256;
 // one round of whole tiles better than two of CTAs (2048 x 10240 x 2048 75 -> 63). Against a CTA per tile pairs have to gain 12 % of the
 // estimate: between other kernels they lose what those gain by starting early (292 x 2048 x 512 in a bf16 encoder 17 -> 21 us; its block of
 // 292 rows 180 us, 183 without the margin, 175 with it). `splits` is how many K slices a CTA per tile would take (linear_tile_choice):
-// left out of the estimate, 256 x 8192 x 512 ran as eight items on pairs in 34 us, its eight slices take 13. Over 583 Linear products of 130 ..
+// left out of the estimate, 256 x 8192 x 512 ran as four items on pairs in 34 us, its eight slices take 13. Over 583 Linear products of 130 ..
 // 4096 rows, 407 of them with slices, each timed on all four, the choice is 1.0 % above the best on average (the worst 3410 x 2632 x 152, 31 us
 // on CTAs, 20 on pairs); over the 407 it was 44 % without the slices' term.
 // HOLO_GEMM_KERNEL names the kernel instead.
